@@ -6,8 +6,9 @@
 // len(a)+len(b)-1 (so it may run Bluestein), real convolution at
 // NextPow2(len(a)+len(b)-1) (at least 2) -- except for long real signals
 // with a short kernel (len(b) - 1 <= L/4 for an L <= 2^15 block and more
-// than two blocks of output), which run overlap-save (k_conv_os): the same
-// linear convolution from single-CTA transforms of 2^12..2^15 points.  The two forward transforms run
+// than two blocks of output), which run overlap-save (k_conv_pair for
+// float32, k_conv_os for float64): the same linear convolution from
+// single-CTA transforms.  The two forward transforms run
 // as one batch of two, the pointwise product is one elementwise kernel
 // (internal/fft/complex_mul.go:23), the inverse writes straight into a
 // padded buffer whose head is the result.  Plans come from a process-wide
@@ -17,6 +18,7 @@
 #include <mutex>
 #include <tuple>
 #include "gfft_internal.h"
+#include "gfft_pairrow.cuh"
 #include "gfft_real.cuh"
 
 namespace gfft {
@@ -212,15 +214,11 @@ cudaError_t launch_conv_os(const void* a, void* dst, int64_t na, int64_t a_dist,
   return cudaGetLastError();
 }
 
-// FFT length of the overlap-save blocks: the smallest power of two with at
-// most an eighth of each window wrapped (L >= 8 (nb - 1)), else at most a
-// quarter, at least 4096, at most what one CTA transforms (2 x 16384
-// complex64, 2 x 8192 complex128); 0 = use one transform of the whole signal
-// (short signals, long kernels).  The longer blocks cost fewer transform
-// points per output and run the transform on more threads per CTA: with a
-// 4097-tap kernel, 2^15-point blocks (28672 outputs each, 512 threads) took
-// 0.45 ms for 64 signals of 2^20 against 0.52 for 2^14-point blocks (12288
-// outputs, 256 threads).
+// Which calls run overlap-save, and the window of the float64 kernel: the
+// smallest power of two with at most an eighth of each window wrapped (L >= 8
+// (nb - 1)), else at most a quarter, at least 4096, at most 2^15 (float64:
+// 2^14, what one CTA transforms as L / 2 complex points); 0 = one transform of
+// the whole signal (short signals, long kernels).
 template <typename R>
 int64_t os_length(int64_t na, int64_t nb) {
   const int64_t lmax = sizeof(R) == 4 ? 32768 : 16384;
@@ -232,27 +230,167 @@ int64_t os_length(int64_t na, int64_t nb) {
   return 0;
 }
 
-template <typename R>
-cudaError_t dispatch_conv_os(int64_t L, const R* a, R* dst, int64_t na, int64_t a_dist, int64_t dst_dist,
+cudaError_t dispatch_conv_os(int64_t L, const double* a, double* dst, int64_t na, int64_t a_dist, int64_t dst_dist,
                              int64_t nout, int64_t nblk, int64_t count, int nb, const void* tw, const void* wt,
                              const void* hs, cudaStream_t st) {
-  using C = Cx<R>;
-  if constexpr (sizeof(R) == 4) {
-    switch (L) {
-      case 4096: return launch_conv_os<C, 2048, 16>(a, dst, na, a_dist, dst_dist, nout, nblk, count, nb, tw, wt, hs, st);
-      case 8192: return launch_conv_os<C, 4096, 16>(a, dst, na, a_dist, dst_dist, nout, nblk, count, nb, tw, wt, hs, st);
-      // 512 threads (16 per thread) ran 1.08x faster than 256 threads (32)
-      case 16384: return launch_conv_os<C, 8192, 16>(a, dst, na, a_dist, dst_dist, nout, nblk, count, nb, tw, wt, hs, st);
-      case 32768: return launch_conv_os<C, 16384, 32>(a, dst, na, a_dist, dst_dist, nout, nblk, count, nb, tw, wt, hs, st);
-    }
-  } else {
-    switch (L) {
-      case 4096: return launch_conv_os<C, 2048, 16>(a, dst, na, a_dist, dst_dist, nout, nblk, count, nb, tw, wt, hs, st);
-      case 8192: return launch_conv_os<C, 4096, 16>(a, dst, na, a_dist, dst_dist, nout, nblk, count, nb, tw, wt, hs, st);
-      case 16384: return launch_conv_os<C, 8192, 16>(a, dst, na, a_dist, dst_dist, nout, nblk, count, nb, tw, wt, hs, st);
-    }
+  using C = double2;
+  switch (L) {
+    case 4096: return launch_conv_os<C, 2048, 16>(a, dst, na, a_dist, dst_dist, nout, nblk, count, nb, tw, wt, hs, st);
+    case 8192: return launch_conv_os<C, 4096, 16>(a, dst, na, a_dist, dst_dist, nout, nblk, count, nb, tw, wt, hs, st);
+    case 16384: return launch_conv_os<C, 8192, 16>(a, dst, na, a_dist, dst_dist, nout, nblk, count, nb, tw, wt, hs, st);
   }
   return cudaErrorInvalidValue;
+}
+
+// ---- float32 overlap-save: two blocks per transform -------------------------
+//
+// Blocks j and j + 1 of one signal (windows of N samples, B = N - (nb - 1) new
+// outputs each) are the real and the imaginary part of one complex transform
+// of N points.  The kernel is real, so its spectrum multiplies both parts
+// alike, and the inverse gives both blocks' outputs: no real-spectrum
+// recombination exists, and the bins never need their natural order -- the
+// inverse runs the forward stages backwards from the registers they end in.
+// Against the half-length form it replaced (recombination of bins k and H - k
+// through shared memory, five table loads per bin) this costs four exchanges
+// through shared memory instead of seven and two table loads per bin pair.
+// The two blocks are neighbours in one signal: their rounding errors mix only
+// with each other's, and no value crosses between signals.
+//
+// Bound: the FMA pipe and the phases of one or a few CTAs per SM.  64 signals
+// of 2^20 with 4097 taps: 0.440 ms before (2^15-sample half-length blocks),
+// 0.291 ms now (N = 16384; FMA pipe busy 43 %), rel-L2 error 7.6e-7 -> 3.1e-7;
+// 32 x 2^20 with 513 taps 0.165 -> 0.094 ms (N = 4096; FMA pipe busy 62 %),
+// one signal of 2^17 with 2049 taps 27.9 -> 12.7 us.
+using ConvRow16k = PairRow<16384, 32, 16, 16>;
+using ConvRow8k = PairRow<8192, 16, 16, 16>;
+using ConvRow4k = PairRow<4096, 16, 16, 8>;
+
+// e in [lo, hi) of a window is a sample of the signal, else zero
+struct PairWindowLoad {
+  const float *a, *b;  // window sample 0 of the two blocks
+  unsigned lo_a, n_a, lo_b, n_b;
+  __device__ __forceinline__ float2 operator()(int e) const {
+    return float2{unsigned(e) - lo_a < n_a ? __ldg(a + e) : 0.f, unsigned(e) - lo_b < n_b ? __ldg(b + e) : 0.f};
+  }
+};
+
+struct PairWindowStore {
+  float *a, *b;  // output of window sample 0 of the two blocks
+  unsigned skip, n_a, n_b;  // the first nb - 1 window samples are wrapped: not outputs
+  __device__ __forceinline__ void operator()(int e, float2 v) const {
+    const unsigned o = unsigned(e) - skip;
+    if (o < n_a) __stcs(a + e, v.x);
+    if (o < n_b) __stcs(b + e, v.y);
+  }
+};
+
+// Spectrum of the kernel, scaled by 1/N, in the register order of
+// K::forward: entry i T + t is pair i of thread t.
+template <typename K>
+__global__ void __launch_bounds__(K::T) k_conv_spectrum(const float* b, int nb, const float2* __restrict__ tw,
+                                                        float4* hs) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float4* sh = reinterpret_cast<float4*>(smem_raw);
+  Pair v[K::EP];
+  K::template forward<-1>(v, sh, threadIdx.x, tw,
+                          [&](int e) { return float2{e < nb ? __ldg(b + e) : 0.f, 0.f}; });
+  const V2 s(1.0 / double(K::N));
+#pragma unroll
+  for (int i = 0; i < K::EP; ++i) K::put(hs, i * K::T + threadIdx.x, Pair{v[i].x * s, v[i].y * s});
+}
+
+__device__ __forceinline__ int64_t clamp_to(int64_t v, int64_t hi) { return v < 0 ? 0 : (v > hi ? hi : v); }
+
+// One CTA per pair of blocks; npair pairs per signal.  ahead > 0: the CTA asks
+// for the samples of CTA blockIdx + ahead to be brought into L2.
+template <typename K, int MINB>
+__global__ void __launch_bounds__(K::T, MINB)
+k_conv_pair(const float* a, float* dst, int64_t na, int64_t a_dist, int64_t dst_dist, int64_t nout, int npair, int nb,
+            const float2* __restrict__ tw, const float4* hs, int ahead) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  float4* sh = reinterpret_cast<float4*>(smem_raw);
+  const int t = threadIdx.x;
+  const int skip = nb - 1, B = K::N - skip;
+  if (ahead > 0 && unsigned(ahead) < gridDim.x - blockIdx.x) {
+    const int g = blockIdx.x + ahead;
+    const int64_t p0 = int64_t(g % npair) * 2 * B - skip;
+    const int64_t lo = clamp_to(p0, na), hi = clamp_to(p0 + B + K::N, na);
+    const float* x = a + (g / npair) * a_dist;
+    const uintptr_t q0 = (reinterpret_cast<uintptr_t>(x + lo) + 15) & ~uintptr_t(15);
+    const uintptr_t q1 = reinterpret_cast<uintptr_t>(x + hi) & ~uintptr_t(15);
+    if (q1 > q0) prefetch_range(reinterpret_cast<const void*>(q0), int64_t(q1 - q0), t, K::T);
+  }
+  const int sig = blockIdx.x / npair;
+  const int64_t pa = int64_t(blockIdx.x % npair) * 2 * B - skip, pb = pa + B;  // window sample 0
+  const float* x = a + sig * a_dist;
+  float* y = dst + sig * dst_dist;
+  Pair v[K::EP];
+  {
+    const int64_t la = clamp_to(-pa, K::N), lb = clamp_to(-pb, K::N);
+    const PairWindowLoad ld{x + pa, x + pb, unsigned(la), unsigned(clamp_to(na - pa - la, K::N - la)), unsigned(lb),
+                            unsigned(clamp_to(na - pb - lb, K::N - lb))};
+    K::template forward<-1>(v, sh, t, tw, ld);
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the kernel's spectrum
+#pragma unroll
+  for (int i = 0; i < K::EP; ++i) v[i] = pmul(v[i], K::get(hs, i * K::T + t));
+  const PairWindowStore st{y + pa, y + pb, unsigned(skip), unsigned(clamp_to(nout - pa - skip, B)),
+                           unsigned(clamp_to(nout - pb - skip, B))};
+  K::template backward<+1>(v, sh, t, tw, st);
+}
+
+template <typename K, int MINB, bool PREFETCH>
+cudaError_t launch_conv_pair(const float* a, float* dst, int64_t na, int64_t a_dist, int64_t dst_dist, int64_t nout,
+                             int64_t count, const float* b, int nb, const float2* tw, float4* hs, cudaStream_t st) {
+  cudaError_t e = raise_smem<&k_conv_spectrum<K>>(K::SMEM);
+  if (e == cudaSuccess) e = raise_smem<&k_conv_pair<K, MINB>>(K::SMEM);
+  if (e != cudaSuccess) return e;
+  static const int64_t resident = resident_ctas(&k_conv_pair<K, MINB>, K::T, K::SMEM);
+  const int64_t B = K::N - (nb - 1), npair = ((nout + B - 1) / B + 1) / 2;
+  if (npair > 0x7fffffffLL / count) return cudaErrorInvalidConfiguration;
+  k_conv_spectrum<K><<<1, K::T, K::SMEM, st>>>(b, nb, tw, hs);
+  e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  // programmatic launch: the forward transforms of the first wave overlap the
+  // one-CTA transform of the kernel
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(count * npair));
+  cfg.blockDim = dim3(K::T);
+  cfg.dynamicSmemBytes = K::SMEM;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, &k_conv_pair<K, MINB>, a, dst, na, a_dist, dst_dist, nout, int(npair), nb, tw,
+                            static_cast<const float4*>(hs), PREFETCH && count * npair > resident ? int(resident) : 0);
+}
+
+// Transform length of the float32 blocks: the one whose waves of CTAs take the
+// least time.  `us` is one full wave (148 SMs x resident CTAs), measured on 64
+// signals of 2^20 (513 taps: 4096 points 0.171, 8192 0.205, 16384 0.261 ms;
+// 4097 taps: 8192 points 0.349, 16384 0.306 ms); a length serves kernels that
+// wrap at most half of its window.  Prefetching the next CTA's samples gained
+// 8 % at 16384 points, 3 % at 8192 and lost 4 % at 4096.
+int os_points(int64_t nout, int64_t count, int64_t nb) {
+  static const struct {
+    int n, resident;
+    double us;
+  } kRows[] = {{4096, 4, 10.7}, {8192, 2, 13.7}, {16384, 1, 16.4}};
+  int best = 16384;
+  double cost = 0;
+  for (const auto& r : kRows) {
+    if (2 * (nb - 1) > r.n) continue;
+    const int64_t B = r.n - (nb - 1), pairs = count * (((nout + B - 1) / B + 1) / 2), wave = 148 * r.resident;
+    const double c = double((pairs + wave - 1) / wave) * r.us;
+    if (cost == 0 || c < cost) {
+      cost = c;
+      best = r.n;
+    }
+  }
+  return best;
 }
 
 }  // namespace
@@ -293,7 +431,31 @@ static gfft_status convolve_real_dev(int prec, R* dst, int64_t dst_dist, const R
   const int64_t L = na + nb - 1;
   // long signals: overlap-save blocks (same linear convolution, transforms
   // of 2^12..2^15 points instead of one of NextPow2(na + nb - 1))
-  if (const int64_t Lb = os_length<R>(na, nb)) {
+  const int64_t Lb = os_length<R>(na, nb);
+  if constexpr (sizeof(R) == 4) {
+    if (Lb) {
+      const int N = os_points(L, count, nb);
+      gfft_plan* tp = nullptr;  // its W_N table
+      gfft_status s = cached_plan(prec, N, &tp);
+      if (s != GFFT_OK) return s;
+      if (tp->core.algo == Algo::Pow2Smem) {
+        float4* hs = nullptr;
+        GFFT_CUDA(ws_alloc(reinterpret_cast<void**>(&hs), size_t(N) * sizeof(float2), st));
+        const float2* tw = static_cast<const float2*>(tp->core.tw);
+        const int64_t dd = count == 1 ? L : dst_dist;
+        cudaError_t e;
+        if (N == 4096)
+          e = launch_conv_pair<ConvRow4k, 4, false>(a, dst, na, a_dist, dd, L, count, b, int(nb), tw, hs, st);
+        else if (N == 8192)
+          e = launch_conv_pair<ConvRow8k, 2, true>(a, dst, na, a_dist, dd, L, count, b, int(nb), tw, hs, st);
+        else
+          e = launch_conv_pair<ConvRow16k, 1, true>(a, dst, na, a_dist, dd, L, count, b, int(nb), tw, hs, st);
+        cudaFreeAsync(hs, st);
+        if (e != cudaSuccess) return cuda_status(e, "k_conv_pair");
+        return GFFT_OK;
+      }
+    }
+  } else if (Lb) {
     gfft_plan_real* bp = nullptr;
     gfft_status s = cached_real_plan(prec, Lb, &bp);
     if (s != GFFT_OK) return s;
@@ -307,8 +469,8 @@ static gfft_status convolve_real_dev(int prec, R* dst, int64_t dst_dist, const R
       if (e == cudaSuccess) s = real_forward(bp, 0, hs, kpad, 1, Lb, hb, st);
       if (e == cudaSuccess && s == GFFT_OK) {
         const int64_t B = Lb - (nb - 1), nblk = (L + B - 1) / B;
-        e = dispatch_conv_os<R>(Lb, a, dst, na, a_dist, count == 1 ? L : dst_dist, L, nblk, count, int(nb),
-                                bp->child.tw, bp->wt, hs, st);
+        e = dispatch_conv_os(Lb, a, dst, na, a_dist, count == 1 ? L : dst_dist, L, nblk, count, int(nb), bp->child.tw,
+                             bp->wt, hs, st);
       }
       cudaFreeAsync(kpad, st);
       if (e != cudaSuccess) return cuda_status(e, "k_conv_os");

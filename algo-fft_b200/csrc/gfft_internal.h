@@ -1,6 +1,7 @@
 // Internal plan object and helpers shared by the C-ABI translation units.
 #pragma once
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -44,6 +45,21 @@ class DeviceGuard {
   int prev_ = 0;
   bool restore_ = false;
 };
+
+// Raises the dynamic shared memory limit of kernel FN to `smem` bytes, once
+// per device (the limit is a property of the function on a device).
+template <auto* FN>
+cudaError_t raise_smem(int smem) {
+  static std::atomic<uint64_t> done{0};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = uint64_t(1) << (dev & 63);
+  if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(FN, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
+}
 
 enum class Algo { Trivial, Pow2Smem, TwoPass, ThreePass, Generic, GenTwoPass, Bluestein, TensorCore, L2Pipe };
 
