@@ -1,19 +1,136 @@
+// Column passes of the multi-pass complex64 transforms on packed column pairs.
+//
+// A tile is NP pairs of adjacent columns of L rows.  Stages are the Stockham
+// stages of the scalar column tiles (same index maps); element (row, pair) is
+// 16 bytes in global and in shared memory, so every access is one 16-byte
+// instruction for two elements and every butterfly one packed instruction.
+//
+// The four-step twiddle is applied where a pass LOADS (the scalar passes apply
+// it where the previous pass stores): its table lookups and products run while
+// the tile's own loads are in flight, and the first pass stores plain columns.
+// Columns leave transposed straight from the last stage's registers: the last
+// stage takes its rows with consecutive threads on consecutive rows of one
+// pair, so a warp stores 256-byte runs of each column and the extra exchange
+// of a transposed store is gone.
 #pragma once
 #include "gfft_pair.cuh"
-namespace gfft {
-enum { PAIR_COLS = 0, PAIR_TWT = 1 };
 
-template <int L, int EPT, int NP, int DIR, int P, int MODE, bool TF, typename LD, typename ST>
-__device__ __forceinline__ void pair_stage(Pair* v, float4* sh, int t, int c, const float2* __restrict__ tw, LD& ld, ST& st) {
+namespace gfft {
+
+// W_N^m from the split table, m < N < 2^32.
+template <int DIR>
+__device__ __forceinline__ float2 pair_twiddle(const BigTwiddle& bt, unsigned m) {
+  const float2* lo = static_cast<const float2*>(bt.lo);
+  const float2* hi = static_cast<const float2*>(bt.hi);
+  float2 w = cmul(__ldg(hi + (m >> bt.shift)), __ldg(lo + (m & ((1u << bt.shift) - 1))));
+  if constexpr (DIR > 0) w.y = -w.y;
+  return w;
+}
+__device__ __forceinline__ Pair two(float2 a, float2 b) { return Pair{V2(float2{a.x, b.x}), V2(float2{a.y, b.y})}; }
+
+// v[r] *= b s^r, r < RS <= 16, from b, s and s4 = s^4 (both rounded from the
+// table, so no factor is more than three products away from it).
+template <int RS>
+__device__ __forceinline__ void pair_scale_powers(Pair* v, Pair b, Pair s, Pair s4) {
+  Pair lo[4];
+  lo[1] = s;
+  if constexpr (RS > 2) lo[2] = pmul(s, s);
+  if constexpr (RS > 3) lo[3] = pmul(lo[2], s);
+  Pair h = b, s8 = s4;
+#pragma unroll
+  for (int j = 0; j < (RS + 3) / 4; ++j) {
+    if (j == 1) h = pmul(b, s4);
+    if (j == 2) {
+      s8 = pmul(s4, s4);
+      h = pmul(b, s8);
+    }
+    if (j == 3) h = pmul(b, pmul(s8, s4));
+#pragma unroll
+    for (int i = 0; i < 4 && 4 * j + i < RS; ++i) v[4 * j + i] = pmul(v[4 * j + i], i == 0 ? h : pmul(h, lo[i]));
+  }
+}
+
+// Load policies: ld(row, c) reads a row of pair c; twiddle(v, t, c) scales the
+// first stage's RS inputs of rows t + r STRIDE.
+struct PairNoTwiddle {
+  template <int RS, int STRIDE, int DIR>
+  __device__ __forceinline__ void twiddle(Pair*, int, int) const {}
+};
+// W_N^(k (a row + b)) for the two columns k = col0 + 2c, + 1
+struct PairColumnTwiddle {
+  BigTwiddle bt;
+  unsigned col0, a, b;
+  template <int RS, int STRIDE, int DIR>
+  __device__ __forceinline__ void twiddle(Pair* v, int t, int c) const {
+    const unsigned k0 = col0 + 2 * c, k1 = k0 + 1, e = a * t + b, es = a * STRIDE;
+    const Pair s4 = RS > 4 ? two(pair_twiddle<DIR>(bt, k0 * es * 4), pair_twiddle<DIR>(bt, k1 * es * 4)) : Pair{};
+    pair_scale_powers<RS>(v, two(pair_twiddle<DIR>(bt, k0 * e), pair_twiddle<DIR>(bt, k1 * e)),
+                          two(pair_twiddle<DIR>(bt, k0 * es), pair_twiddle<DIR>(bt, k1 * es)), s4);
+  }
+};
+// W_M^(k row) for one k and every column of the tile
+struct PairRowTwiddle {
+  BigTwiddle bt;
+  unsigned k;
+  template <int RS, int STRIDE, int DIR>
+  __device__ __forceinline__ void twiddle(Pair* v, int t, int) const {
+    const Pair s4 = RS > 4 ? pbroadcast(pair_twiddle<DIR>(bt, k * STRIDE * 4)) : Pair{};
+    pair_scale_powers<RS>(v, pbroadcast(pair_twiddle<DIR>(bt, k * t)), pbroadcast(pair_twiddle<DIR>(bt, k * STRIDE)),
+                          s4);
+  }
+};
+
+template <typename TW, bool CG>
+struct PairLoad : TW {
+  const float2* in;  // row 0, column 0 of the tile
+  int64_t pitch;
+  __device__ __forceinline__ Pair operator()(int row, int c) const {
+    const float4* p = reinterpret_cast<const float4*>(in + row * pitch) + c;
+    return pair_of(CG ? __ldcg(p) : __ldcs(p));
+  }
+};
+
+// Store policies: ROWS_FIRST takes the last stage's rows with consecutive
+// threads on consecutive rows of one pair.
+template <bool SCALE, bool CG>
+struct PairStoreRows {
+  static constexpr bool ROWS_FIRST = false;
+  float2* out;
+  int64_t pitch;
+  float scale;
+  __device__ __forceinline__ void operator()(int row, int c, Pair o) const {
+    if constexpr (SCALE) {
+      const V2 s(float2{scale, scale});
+      o = Pair{o.x * s, o.y * s};
+    }
+    float4* p = reinterpret_cast<float4*>(out + row * pitch) + c;
+    if constexpr (CG) __stcg(p, pair_raw(o));
+    else __stcs(p, pair_raw(o));
+  }
+};
+// column c of the tile as a row of `pitch` elements
+struct PairStoreTransposed {
+  static constexpr bool ROWS_FIRST = true;
+  float2* out;  // of column 0
+  int64_t pitch;
+  __device__ __forceinline__ void operator()(int row, int c, Pair o) const {
+    float2* p = out + 2 * c * pitch + row;
+    __stcg(p, float2{o.x.v.x, o.y.v.x});
+    __stcg(p + pitch, float2{o.x.v.y, o.y.v.y});
+  }
+};
+
+template <int L, int EPT, int NP, int DIR, int P, typename LD, typename ST>
+__device__ __forceinline__ void pair_stage(Pair* v, float4* sh, int t, int c, const float2* __restrict__ tw,
+                                           const LD& ld, const ST& st) {
   using S = PairShape<L, EPT, NP>;
   using SC = Sched<L, EPT>;
   constexpr int T = S::T, RS = SC::radix_at(P), Q = EPT / RS, STRIDE = L / RS;
   constexpr bool FIRST = P == 1, LAST = P * RS == L;
-  if constexpr (LAST && TF) {  // whole columns per warp from here on
+  if constexpr (LAST && ST::ROWS_FIRST) {
     t = threadIdx.x % T;
     c = threadIdx.x / T;
   }
-  if constexpr (LAST) st.template begin<Q, T, P>(t, c);
   if constexpr (FIRST) {
 #pragma unroll
     for (int q = 0; q < Q; ++q)
@@ -30,16 +147,20 @@ __device__ __forceinline__ void pair_stage(Pair* v, float4* sh, int t, int c, co
   }
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
-    if constexpr (P > 1) {
-      const int k = (t + q * T) & (P - 1);
+    if constexpr (FIRST) {
+      ld.template twiddle<RS, STRIDE, DIR>(v + q * RS, t + q * T, c);
+    } else {
       PairPowers<RS> pw;
-      pw.template load<DIR>(tw, k * (L / (P * RS)));
+      pw.template load<DIR>(tw, ((t + q * T) & (P - 1)) * (L / (P * RS)));
       pw.apply(v + q * RS);
     }
     pdft<RS, DIR>(v + q * RS);
   }
   if constexpr (LAST) {
-    st.template finish<Q, RS, T, P>(v, t, c);
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+#pragma unroll
+      for (int r = 0; r < RS; ++r) st(t + q * T + r * P, c, v[q * RS + r]);
   } else {
     if constexpr (!FIRST) __syncthreads();
 #pragma unroll
@@ -52,86 +173,74 @@ __device__ __forceinline__ void pair_stage(Pair* v, float4* sh, int t, int c, co
       }
     }
     __syncthreads();
-    pair_stage<L, EPT, NP, DIR, P * RS, MODE, TF>(v, sh, t, c, tw, ld, st);
+    pair_stage<L, EPT, NP, DIR, P * RS>(v, sh, t, c, tw, ld, st);
   }
 }
 
-template <bool CG> struct PairLoad {
-  const float2* in; int64_t pitch;
-  __device__ __forceinline__ Pair operator()(int row, int c) const {
-    const float4* p = reinterpret_cast<const float4*>(in + row * pitch) + c;
-    return pair_of(CG ? __ldcg(p) : __ldcs(p));
-  }
-};
-template <int DIR> struct PairStoreCols {
-  float2* out; int64_t pitch; float scale;
-  template <int Q, int T, int P> __device__ __forceinline__ void begin(int, int) {}
-  template <int Q, int RS, int T, int P> __device__ __forceinline__ void finish(Pair* v, int t, int c) {
-#pragma unroll
-    for (int q = 0; q < Q; ++q)
-#pragma unroll
-      for (int r = 0; r < RS; ++r) {
-        Pair o = v[q * RS + r];
-        if constexpr (DIR > 0) { const V2 s(float2{scale, scale}); o = Pair{o.x * s, o.y * s}; }
-        __stcs(reinterpret_cast<float4*>(out + int64_t(t + q * T + r * P) * pitch) + c, pair_raw(o));
-      }
-  }
-};
-// times W_N^{n2 k1}, stored as rows of length N1: Y[n2][k1]
-template <int DIR> struct PairStoreTwT {
-  float2* y; int64_t n1; int col0; BigTwiddle bt;
-  float2 s0, s1, b0[16], b1[16];
-  template <int Q, int T, int P> __device__ __forceinline__ void begin(int t, int c) {
-    const int64_t m = col0 + 2 * c;
-    s0 = big_twiddle<float2, DIR>(bt, m * P); s1 = big_twiddle<float2, DIR>(bt, (m + 1) * P);
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      b0[q] = big_twiddle<float2, DIR>(bt, m * (t + q * T)); b1[q] = big_twiddle<float2, DIR>(bt, (m + 1) * (t + q * T));
-    }
-  }
-  template <int Q, int RS, int T, int P> __device__ __forceinline__ void finish(Pair* v, int t, int c) {
-    Pair pw[RS];
-    pw[1] = (Pair{V2(float2{s0.x, s1.x}), V2(float2{s0.y, s1.y})});
-#pragma unroll
-    for (int r = 2; r < RS; ++r) pw[r] = pmul(pw[r / 2], pw[r - r / 2]);
-    float2* y0 = y + int64_t(col0 + 2 * c) * n1;
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const Pair b = (Pair{V2(float2{b0[q].x, b1[q].x}), V2(float2{b0[q].y, b1[q].y})});
-#pragma unroll
-      for (int r = 0; r < RS; ++r) {
-        const Pair o = pmul(v[q * RS + r], r == 0 ? b : pmul(b, pw[r]));
-        const int row = t + q * T + r * P;
-        __stcg(y0 + row, float2{o.x.v.x, o.y.v.x});
-        __stcg(y0 + n1 + row, float2{o.x.v.y, o.y.v.y});
-      }
-    }
-  }
-};
-struct PairParams { const float2* src; float2* dst; float2* scratch; int64_t idist, odist; const float2* tw1; const float2* tw2; BigTwiddle bt; float scale; };
-
-template <int N1, int N2, int EPT, int NP, int DIR, bool TF, int MINB>
-__global__ void __launch_bounds__(PairShape<N1, EPT, NP>::TPB, MINB) k_pair1(PairParams p) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  float4* sh = reinterpret_cast<float4*>(smem_raw);
-  constexpr int TILES = N2 / (2 * NP);
-  const int64_t bl = blockIdx.x / TILES;
-  const int col0 = int(blockIdx.x % TILES) * 2 * NP;
-  PairLoad<false> ld{p.src + bl * p.idist + col0, N2};
-  PairStoreTwT<DIR> st; st.y = p.scratch + bl * int64_t(N1) * N2; st.n1 = N1; st.col0 = col0; st.bt = p.bt;
+template <int L, int EPT, int NP, int DIR, typename LD, typename ST>
+__device__ __forceinline__ void pair_columns(float4* sh, const float2* __restrict__ tw, const LD& ld, const ST& st) {
   Pair v[EPT];
-  pair_stage<N1, EPT, NP, DIR, 1, PAIR_TWT, TF>(v, sh, threadIdx.x / NP, threadIdx.x % NP, p.tw1, ld, st);
+  pair_stage<L, EPT, NP, DIR, 1>(v, sh, threadIdx.x / NP, threadIdx.x % NP, tw, ld, st);
+}
+
+struct PairPassParams {
+  const float2* src;
+  float2* dst;
+  float2* scratch;
+  int64_t idist, odist;
+  const float2 *tw1, *tw2, *tw3;  // W_L of the passes
+  BigTwiddle bt, btm;             // W_N, W_M (three passes)
+  float scale;
+};
+
+// Two passes, N = N1 N2: Y[n2][k1] = columns of x; X[k1 + N1 k2] = columns of Y
+// x W_N^(n2 k1).  One tile per CTA, tiles of a transform adjacent.
+template <int N1, int N2, int EPT, int NP, int DIR, int MINB>
+__global__ void __launch_bounds__(PairShape<N1, EPT, NP>::TPB, MINB) k_pair_tp1(PairPassParams p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int TILES = N2 / (2 * NP);
+  const int64_t b = blockIdx.x / TILES;
+  const int col0 = int(blockIdx.x % TILES) * 2 * NP;
+  const PairLoad<PairNoTwiddle, false> ld{{}, p.src + b * p.idist + col0, N2};
+  const PairStoreTransposed st{p.scratch + b * (int64_t(N1) * N2) + int64_t(col0) * N1, N1};
+  pair_columns<N1, EPT, NP, DIR>(reinterpret_cast<float4*>(smem_raw), p.tw1, ld, st);
 }
 template <int N1, int N2, int EPT, int NP, int DIR, int MINB>
-__global__ void __launch_bounds__(PairShape<N2, EPT, NP>::TPB, MINB) k_pair2(PairParams p) {
+__global__ void __launch_bounds__(PairShape<N2, EPT, NP>::TPB, MINB) k_pair_tp2(PairPassParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float4* sh = reinterpret_cast<float4*>(smem_raw);
   constexpr int TILES = N1 / (2 * NP);
-  const int64_t bl = blockIdx.x / TILES;
+  const int64_t b = blockIdx.x / TILES;
   const int col0 = int(blockIdx.x % TILES) * 2 * NP;
-  PairLoad<true> ld{p.scratch + bl * int64_t(N1) * N2 + col0, N1};
-  PairStoreCols<DIR> st{p.dst + bl * p.odist + col0, N1, p.scale};
-  Pair v[EPT];
-  pair_stage<N2, EPT, NP, DIR, 1, PAIR_COLS, false>(v, sh, threadIdx.x / NP, threadIdx.x % NP, p.tw2, ld, st);
+  const PairLoad<PairColumnTwiddle, true> ld{{p.bt, unsigned(col0), 1, 0},
+                                             p.scratch + b * (int64_t(N1) * N2) + col0, N1};
+  const PairStoreRows<(DIR > 0), false> st{p.dst + b * p.odist + col0, N1, p.scale};
+  pair_columns<N2, EPT, NP, DIR>(reinterpret_cast<float4*>(smem_raw), p.tw2, ld, st);
 }
+
+// Three passes, N = N1 M, M = M1 M2 (index maps of k_tp3): pass 1 as above
+// with N2 = M; pass 2 over m1, in place on Y[M2 m1 + m2][k1] x W_N^(m k1);
+// pass 3 over m2, x W_M^(m2 k'1), natural order.
+template <int N1, int M1, int M2, int EPT, int NP, int DIR, int MINB>
+__global__ void __launch_bounds__(PairShape<M1, EPT, NP>::TPB, MINB) k_pair_tp3b(PairPassParams p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int G = N1 / (2 * NP), TILES = M2 * G;
+  const int64_t b = blockIdx.x / TILES;
+  const int r = int(blockIdx.x % TILES), m2 = r / G, col0 = (r % G) * 2 * NP;
+  float2* y = p.scratch + b * (int64_t(N1) * M1 * M2) + int64_t(m2) * N1 + col0;
+  const PairLoad<PairColumnTwiddle, true> ld{{p.bt, unsigned(col0), unsigned(M2), unsigned(m2)}, y, int64_t(M2) * N1};
+  const PairStoreRows<false, true> st{y, int64_t(M2) * N1, 1.f};
+  pair_columns<M1, EPT, NP, DIR>(reinterpret_cast<float4*>(smem_raw), p.tw2, ld, st);
 }
+template <int N1, int M1, int M2, int EPT, int NP, int DIR, int MINB>
+__global__ void __launch_bounds__(PairShape<M2, EPT, NP>::TPB, MINB) k_pair_tp3c(PairPassParams p) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int G = N1 / (2 * NP), TILES = M1 * G;
+  const int64_t b = blockIdx.x / TILES;
+  const int r = int(blockIdx.x % TILES), k1 = r / G, col0 = (r % G) * 2 * NP;
+  const PairLoad<PairRowTwiddle, true> ld{{p.btm, unsigned(k1)},
+                                          p.scratch + b * (int64_t(N1) * M1 * M2) + int64_t(M2) * k1 * N1 + col0, N1};
+  const PairStoreRows<(DIR > 0), false> st{p.dst + b * p.odist + int64_t(N1) * k1 + col0, int64_t(N1) * M1, p.scale};
+  pair_columns<M2, EPT, NP, DIR>(reinterpret_cast<float4*>(smem_raw), p.tw3, ld, st);
+}
+
+}  // namespace gfft

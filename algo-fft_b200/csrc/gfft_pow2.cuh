@@ -150,12 +150,14 @@ inline int64_t resident_ctas(F* fn, int tpb, int smem) {
   return int64_t(sms) * (occ > 0 ? occ : 1);
 }
 
-template <typename C>
+template <typename C, bool EVICT = false>
 struct GlobalLoad {
   static constexpr bool kShared = false;
   const C* in;
   bool valid;
-  __device__ __forceinline__ C operator()(int e) const { return valid ? ld_stream(in + e) : C{0, 0}; }
+  __device__ __forceinline__ C operator()(int e) const {
+    return !valid ? C{0, 0} : EVICT ? ld_evict(in + e) : ld_stream(in + e);
+  }
 };
 
 template <typename C, bool SCALE>
@@ -213,7 +215,7 @@ k_pow2(const C* src, C* dst, int64_t count, int64_t idist, int64_t odist, const 
       static_assert((1 << LN) == N, "staged I/O covers N <= 256");
       const C* in = src + b0 * N;
       for (int e = threadIdx.x; e < nb * N; e += S::TPB)
-        shc[(e >> LN) * S::STRIDE + S::pad(e & (N - 1))] = ld_stream(in + e);
+        shc[(e >> LN) * S::STRIDE + S::pad(e & (N - 1))] = ld_evict(in + e);
       __syncthreads();
       RowShared<C, N, EPT> io{sh};
       pow2_fft<C, N, EPT, DIR>(sh, t, tw, io, io);
@@ -227,7 +229,7 @@ k_pow2(const C* src, C* dst, int64_t count, int64_t idist, int64_t odist, const 
       return;
     }
   }
-  GlobalLoad<C> ld{src + (valid ? b * idist : 0), valid};
+  GlobalLoad<C, true> ld{src + (valid ? b * idist : 0), valid};
   GlobalStore<C, (DIR > 0)> st{dst + (valid ? b * odist : 0), valid, scale};
   pow2_fft<C, N, EPT, DIR>(sh, t, tw, ld, st);
 }

@@ -57,7 +57,7 @@ struct ColShape {
 
 // LOAD_SMEM: the tile is already in shared memory (a TMA copy put it there).
 // LOAD_FN: the first stage asks the caller's IO object, io.load(row, c).
-enum { LOAD_STREAM = 0, LOAD_L2 = 1, LOAD_SMEM = 2, LOAD_FN = 3 };
+enum { LOAD_STREAM = 0, LOAD_L2 = 1, LOAD_SMEM = 2, LOAD_FN = 3, LOAD_EVICT = 4 };
 // OUT_SMEM: the result, scaled, back into the tile's rows (for a TMA store);
 // OUT_SMEM_TWIDDLE_T: times the big twiddle, transposed into rows of L + 1
 // elements per column, for a coalesced store of whole columns.
@@ -87,6 +87,7 @@ __device__ __forceinline__ int swz128(int row, int c) {
 template <int LOADK, typename C>
 __device__ __forceinline__ C gload(const C* p) {
   if constexpr (LOADK == LOAD_L2) return __ldcg(p);
+  else if constexpr (LOADK == LOAD_EVICT) return ld_evict(p);
   else return ld_stream(p);
 }
 

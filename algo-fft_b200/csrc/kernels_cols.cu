@@ -41,7 +41,7 @@ k_pow2_cols(const C* src, C* dst, int64_t ncols, int64_t pitch, int64_t dist, in
   C* out = dst + arr * dist + col0;
   const BigTwiddle bt{nullptr, nullptr, 0};
   C v[T::EPT];
-  col_stage<C, L, T::EPT, T::NC, DIR, 1, LOAD_STREAM, OUT_COLUMNS, 0, 0>(v, in, out, sh, t, c, active, tw, scale, bt,
+  col_stage<C, L, T::EPT, T::NC, DIR, 1, LOAD_EVICT, OUT_COLUMNS, 0, 0>(v, in, out, sh, t, c, active, tw, scale, bt,
                                                                          0, pitch);
 }
 
