@@ -9,6 +9,7 @@
 #include "gfft_internal.h"
 #include "gfft_math.cuh"
 #include "gfft_l2pipe.cuh"
+#include "gfft_pairpass.cuh"
 #include "gfft_threepass.cuh"
 #include "gfft_twopass.cuh"
 
@@ -243,19 +244,31 @@ static int default_ept(int prec, int64_t n) {
 static std::string twopass_token(const TwoPassKernel* k);
 static std::string threepass_token(const ThreePassKernel* k);
 
+// W_N^(k P), W_N^(4 k P), k < N / N1, of a packed-pair plan.
+static gfft_status fill_pair_tables(PlanCore* c, const PairKernel* k, void* where) {
+  const int64_t m = c->n / k->n1;
+  c->pair_tw = where;
+  c->pair = k;
+  const gfft_status s = fill_twiddles(kC64, where, c->n, m, k->prefix, 0);
+  return s != GFFT_OK ? s : fill_twiddles(kC64, static_cast<float2*>(where) + m, c->n, m, 4 * k->prefix, 0);
+}
+
 // Two-pass plan: tables W_N1, W_N2 and the split table of W_N in one
 // allocation; slot geometry sized so the live intermediate stays in L2.
-static gfft_status init_twopass(PlanCore* c, const TwoPassKernel* f, const TwoPassKernel* inv) {
+static gfft_status init_twopass(PlanCore* c, const TwoPassKernel* f, const TwoPassKernel* inv,
+                                const PairKernel* pair = nullptr) {
   const int64_t n = c->n, n1 = f->n1, n2 = f->n2;
   const size_t es = elem_bytes(c->prec);
   int shift = (ilog2(n) + 1) / 2;
   const int64_t nlo = int64_t(1) << shift, nhi = n >> shift;
-  GFFT_CUDA(cudaMalloc(&c->tw, size_t(n1 + n2 + nlo + nhi) * es));
+  const int64_t base_len = n1 + n2 + nlo + nhi;  // even: the pair tables stay 16-byte aligned
+  GFFT_CUDA(cudaMalloc(&c->tw, size_t(base_len + (pair ? 2 * n2 : 0)) * es));
   char* base = static_cast<char*>(c->tw);
   gfft_status s = fill_twiddles(c->prec, base, n1, n1, 1, 0);
   if (s == GFFT_OK) s = fill_twiddles(c->prec, base + n1 * es, n2, n2, 1, 0);
   if (s == GFFT_OK) s = fill_twiddles(c->prec, base + (n1 + n2) * es, n, nlo, 1, 0);
   if (s == GFFT_OK) s = fill_twiddles(c->prec, base + (n1 + n2 + nlo) * es, n, nhi, nlo, 0);
+  if (s == GFFT_OK && pair) s = fill_pair_tables(c, pair, base + base_len * es);
   if (s != GFFT_OK) return s;
   GFFT_CUDA(cudaStreamSynchronize(0));
   c->tp[0] = f;
@@ -314,13 +327,14 @@ static gfft_status init_l2pipe(PlanCore* c, const L2PipeKernel* f, const L2PipeK
 
 // Three-pass plan: W_N1 | W_M1 | W_M2 | split W_N | split W_M in one
 // allocation.
-static gfft_status init_threepass(PlanCore* c, const ThreePassKernel* f, const ThreePassKernel* inv) {
+static gfft_status init_threepass(PlanCore* c, const ThreePassKernel* f, const ThreePassKernel* inv,
+                                  const PairKernel* pair = nullptr) {
   const int64_t n = c->n, n1 = f->n1, m1 = f->m1, m2 = f->m2, m = m1 * m2;
   const size_t es = elem_bytes(c->prec);
   const int shn = (ilog2(n) + 1) / 2, shm = (ilog2(m) + 1) / 2;
   const int64_t nlo = int64_t(1) << shn, nhi = n >> shn, mlo = int64_t(1) << shm, mhi = m >> shm;
   const int64_t total = n1 + m1 + m2 + nlo + nhi + mlo + mhi;
-  GFFT_CUDA(cudaMalloc(&c->tw, size_t(total) * es));
+  GFFT_CUDA(cudaMalloc(&c->tw, size_t(total + (pair ? 2 * m : 0)) * es));
   char* base = static_cast<char*>(c->tw);
   int64_t off = 0;
   auto put = [&](int64_t len, int64_t cnt, int64_t step, const void** where) -> gfft_status {
@@ -336,6 +350,7 @@ static gfft_status init_threepass(PlanCore* c, const ThreePassKernel* f, const T
   if (s == GFFT_OK) s = put(n, nhi, nlo, &c->bt_hi);
   if (s == GFFT_OK) s = put(m, mlo, 1, &c->btm_lo);
   if (s == GFFT_OK) s = put(m, mhi, mlo, &c->btm_hi);
+  if (s == GFFT_OK && pair) s = fill_pair_tables(c, pair, base + total * es);  // total is even
   if (s != GFFT_OK) return s;
   GFFT_CUDA(cudaStreamSynchronize(0));
   c->bt_shift = shn;
@@ -346,6 +361,34 @@ static gfft_status init_threepass(PlanCore* c, const ThreePassKernel* f, const T
   c->t3[1] = inv;
   c->algo = Algo::ThreePass;
   c->name = threepass_token(f);
+  return GFFT_OK;
+}
+
+// Token of a packed-pair plan: the scalar schedule it falls back to, "-pair".
+static std::string pair_token(const PairKernel* k) {
+  std::string t = std::string(k->m2 ? "gpu-sm100-tp3-" : "gpu-sm100-tp-") + std::to_string(k->n1) + "x" +
+                  std::to_string(k->m1);
+  if (k->m2) return t + "x" + std::to_string(k->m2) + "-pair";
+  return t + "-t" + std::to_string(k->te) + "-e" + std::to_string(k->emax) + "-pair";
+}
+
+// Two- or three-pass plan on the packed-pair kernels.
+static gfft_status init_pair(PlanCore* c, const PairKernel* k) {
+  gfft_status s = GFFT_ERR_NOT_IMPLEMENTED;
+  if (k->m2) {
+    const ThreePassKernel* f = find_threepass(c->prec, c->n, -1);
+    const ThreePassKernel* i = find_threepass(c->prec, c->n, +1);
+    if (f && i && f->n1 == k->n1 && f->m1 == k->m1) s = init_threepass(c, f, i, k);
+  } else {
+    const TwoPassKernel* f = find_twopass(c->prec, c->n, -1, k->te, k->emax);
+    const TwoPassKernel* i = find_twopass(c->prec, c->n, +1, k->te, k->emax);
+    if (f && i && f->n1 == k->n1) s = init_twopass(c, f, i, k);
+  }
+  if (s != GFFT_OK) {
+    if (s == GFFT_ERR_NOT_IMPLEMENTED) set_error("no scalar kernels of the packed-pair split");
+    return s;
+  }
+  c->name = pair_token(k);
   return GFFT_OK;
 }
 
@@ -374,6 +417,7 @@ std::vector<std::string> variant_tokens(int prec, int64_t n) {
     for (const L2PipeKernel* k : l2pipe_variants(prec, n, -1))
       for (int gmb : {8, 16}) v.push_back(l2pipe_token(k, gmb));
     for (const ThreePassKernel* k : threepass_variants(prec, n, -1)) v.push_back(threepass_token(k));
+    if (const PairKernel* k = prec == kC64 ? find_pair(n) : nullptr) v.push_back(pair_token(k));
   } else if (n > 1 && is_smooth7(n)) {
     // runtime-radix schedules (single CTA when it fits, two passes when n
     // has a 7-smooth divisor >= 2 below sqrt n) against Bluestein
@@ -415,6 +459,8 @@ gfft_status core_init_variant(PlanCore* c, int prec, int64_t n, int device, cons
   c->device = device;
   GFFT_CUDA(prepare_kernels());
   int a = 0, b = 0, te = 0, e = 0;
+  if (const PairKernel* k = prec == kC64 ? find_pair(n) : nullptr)
+    if (tok == pair_token(k)) return init_pair(c, k);
   if (std::sscanf(tok.c_str(), "gpu-sm100-p2-n%d-e%d", &a, &e) == 2 && a == n) return init_pow2(c, e);
   if (std::sscanf(tok.c_str(), "gpu-sm100-tp-%dx%d-t%d-e%d", &a, &b, &te, &e) == 4 && int64_t(a) * b == n) {
     const TwoPassKernel* f = find_twopass(prec, n, -1, te, e);
@@ -540,6 +586,9 @@ gfft_status core_init(PlanCore* c, int prec, int64_t n, int device, int strategy
   const bool want_single = strategy == GFFT_KERNEL_DIT || strategy == GFFT_KERNEL_STOCKHAM;
   const bool want_bluestein = strategy == GFFT_KERNEL_BLUESTEIN;
   if (pow2 && n <= max_single && !want_twopass && !want_bluestein) return init_pow2(c, default_ept(prec, n));
+  if (pow2 && prec == kC64 && !want_single && !want_bluestein) {
+    if (const PairKernel* k = find_pair(n)) return init_pair(c, k);
+  }
   if (pow2 && !want_single && strategy != GFFT_KERNEL_BLUESTEIN) {
     const TwoPassKernel* f = find_twopass(prec, n, -1, prec == kC64 ? 8192 : 4096, prec == kC64 ? 16 : 8);
     const TwoPassKernel* i = find_twopass(prec, n, +1, prec == kC64 ? 8192 : 4096, prec == kC64 ? 16 : 8);
@@ -593,19 +642,20 @@ void core_free(PlanCore* c) {
   c->mixc = false;
   c->mixr = false;
   c->bsm = false;
+  c->pair = nullptr;
+  c->pair_tw = nullptr;
   c->algo = Algo::Trivial;
 }
 
-// Two-pass execution in the split schedule (k_tp_split): per chunk of up to
-// 1 GiB of intermediate, one pass-1 launch and one pass-2 launch.  The
-// scratch comes from the library's workspace pool.
-static gfft_status exec_twopass(const PlanCore* c, int dir, void* dst, const void* src, int64_t count,
-                                int64_t idist, int64_t odist, cudaStream_t st) {
-  const TwoPassKernel* k = c->tp[dir < 0 ? 0 : 1];
-  const int64_t tbytes = c->n * int64_t(elem_bytes(c->prec));
-  const int64_t nb = std::max<int64_t>(1, std::min<int64_t>(count, (int64_t(1) << 30) / tbytes));
-  void* ws = nullptr;
-  GFFT_CUDA(ws_alloc(reinterpret_cast<void**>(&ws), size_t(nb) * size_t(tbytes), st));
+// The packed-pair kernels read and write 16 bytes: two adjacent elements.
+static bool pair_aligned(const void* dst, const void* src, int64_t idist, int64_t odist) {
+  return ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0 && idist % 2 == 0 &&
+         odist % 2 == 0;
+}
+
+// Parameters of the scalar two-pass kernels of a plan.
+static TwoPassParams twopass_params(const PlanCore* c, int dir, void* dst, const void* src, void* ws, int64_t count,
+                                    int64_t idist, int64_t odist) {
   TwoPassParams p{};
   p.src = src;
   p.dst = dst;
@@ -621,6 +671,61 @@ static gfft_status exec_twopass(const PlanCore* c, int dir, void* dst, const voi
   p.scale = dir < 0 ? 1.0 : 1.0 / double(c->n);
   p.status = c->status;
   p.spin_limit = 1u << 22;
+  return p;
+}
+
+// Packed-pair execution: per chunk of up to 1 GiB of intermediate, one launch
+// per pass.
+static gfft_status exec_pair(const PlanCore* c, int dir, void* dst, const void* src, int64_t count, int64_t idist,
+                             int64_t odist, cudaStream_t st) {
+  const PairKernel* k = c->pair;
+  const int d = dir < 0 ? 0 : 1;
+  const int64_t tbytes = c->n * int64_t(sizeof(float2)), m1 = c->n / k->n1;
+  const int64_t nb = std::max<int64_t>(1, std::min<int64_t>(count, (int64_t(1) << 30) / tbytes));
+  void* ws = nullptr;
+  GFFT_CUDA(ws_alloc(&ws, size_t(nb) * size_t(tbytes), st));
+  PairPassParams p{};
+  p.scratch = static_cast<float2*>(ws);
+  p.idist = idist;
+  p.odist = odist;
+  p.tw1 = static_cast<const float2*>(c->tw1);
+  p.tw2 = static_cast<const float2*>(c->tw2);
+  p.tw3 = static_cast<const float2*>(c->tw3);
+  p.bt = BigTwiddle{c->bt_lo, c->bt_hi, c->bt_shift};
+  p.btm = BigTwiddle{c->btm_lo, c->btm_hi, c->btm_shift};
+  p.ts = static_cast<const float2*>(c->pair_tw);
+  p.ts4 = p.ts + m1;
+  p.scale = dir < 0 ? 1.f : float(1.0 / double(c->n));
+  const TwoPassParams sp =
+      k->first_only ? twopass_params(c, dir, dst, src, ws, count, idist, odist) : TwoPassParams{};
+  cudaError_t e = cudaSuccess;
+  for (int64_t b0 = 0; b0 < count && e == cudaSuccess; b0 += nb) {
+    const int64_t m = std::min(nb, count - b0);
+    p.src = static_cast<const float2*>(src) + b0 * idist;
+    p.dst = static_cast<float2*>(dst) + b0 * odist;
+    e = k->launch[d](p, 1, m, st);
+    if (k->first_only) {
+      if (e == cudaSuccess) e = c->tp[d]->split(sp, 2, b0, m, st);
+      continue;
+    }
+    for (int pass = 2; pass <= (k->m2 ? 3 : 2) && e == cudaSuccess; ++pass) e = k->launch[d](p, pass, m, st);
+  }
+  cudaFreeAsync(ws, st);
+  if (e != cudaSuccess) return cuda_status(e, "k_pair");
+  return GFFT_OK;
+}
+
+// Two-pass execution in the split schedule (k_tp_split): per chunk of up to
+// 1 GiB of intermediate, one pass-1 launch and one pass-2 launch.  The
+// scratch comes from the library's workspace pool.
+static gfft_status exec_twopass(const PlanCore* c, int dir, void* dst, const void* src, int64_t count,
+                                int64_t idist, int64_t odist, cudaStream_t st) {
+  const TwoPassKernel* k = c->tp[dir < 0 ? 0 : 1];
+  const int64_t tbytes = c->n * int64_t(elem_bytes(c->prec));
+  const int64_t nb = std::max<int64_t>(1, std::min<int64_t>(count, (int64_t(1) << 30) / tbytes));
+  void* ws = nullptr;
+  GFFT_CUDA(ws_alloc(reinterpret_cast<void**>(&ws), size_t(nb) * size_t(tbytes), st));
+  const TwoPassParams p = twopass_params(c, dir, dst, src, ws, count, idist, odist);
   cudaError_t e = cudaSuccess;
   for (int64_t b0 = 0; b0 < count && e == cudaSuccess; b0 += nb) {
     const int64_t m = std::min(nb, count - b0);
@@ -731,10 +836,12 @@ gfft_status core_exec(const PlanCore* c, int dir, void* dst, const void* src, in
       return GFFT_OK;
     }
     case Algo::TwoPass:
+      if (c->pair && pair_aligned(dst, src, idist, odist)) return exec_pair(c, dir, dst, src, count, idist, odist, st);
       return exec_twopass(c, dir, dst, src, count, idist, odist, st);
     case Algo::L2Pipe:
       return exec_l2pipe(c, dir, dst, src, count, idist, odist, st);
     case Algo::ThreePass:
+      if (c->pair && pair_aligned(dst, src, idist, odist)) return exec_pair(c, dir, dst, src, count, idist, odist, st);
       return exec_threepass(c, dir, dst, src, count, idist, odist, st);
     case Algo::Generic:
     case Algo::GenTwoPass:

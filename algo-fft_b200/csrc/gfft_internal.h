@@ -83,6 +83,10 @@ struct PlanCore {
   const void* btm_lo = nullptr;
   const void* btm_hi = nullptr;
   int btm_shift = 0;
+  // packed-pair kernels of a two- or three-pass schedule, for 16-byte aligned
+  // buffers (null: not chosen), and their tables W_N^(k P), W_N^(4 k P)
+  const PairKernel* pair = nullptr;
+  const void* pair_tw = nullptr;  // in tw
   const void* tw1 = nullptr;                     // W_N1
   const void* tw2 = nullptr;                     // W_N2
   const void* bt_lo = nullptr;

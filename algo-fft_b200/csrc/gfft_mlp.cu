@@ -267,6 +267,7 @@ static bool plan_features(int prec, int64_t n, int64_t batch, int64_t stride, in
   f[9] = float(real ? 1 : 0);
   int a = 0, b = 0, te = 0, e = 0, ns = 0, l = 0;
   long long l1 = 0, l2 = 0, ln = 0;
+  if (tok.size() > 5 && tok.compare(tok.size() - 5, 5, "-pair") == 0) return false;  // no features: not in the data
   if (std::sscanf(tok.c_str(), "gpu-sm100-p2-n%d-e%d", &a, &e) == 2) {
     f[10] = 1.f;
     f[14] = float(ilog2f(e));

@@ -54,6 +54,18 @@ struct L2PipeKernel {
   cudaError_t (*launch)(const L2pParams& p, cudaStream_t st);
 };
 
+// Packed-pair kernels of a complex64 length: two passes N1 x M1 (m2 = 0) or
+// three N1 x M1 x M2.  te / emax name the scalar two-pass tile that serves
+// buffers the 16-byte accesses cannot (three passes: the plain k_tp3).
+struct PairPassParams;
+struct PairKernel {
+  int n1, m1, m2, te, emax;
+  int prefix;       // prefix product of pass 1's last stage (the step of its tables)
+  bool first_only;  // two passes: the second is the scalar tile's
+  cudaError_t (*launch[2])(const PairPassParams& p, int pass, int64_t nb, cudaStream_t st);  // forward, inverse
+};
+const PairKernel* find_pair(int64_t n);
+
 void register_l2pipe(const L2PipeKernel& k);
 // The variant of this shape and direction; nc1 = 0 takes the first registered.
 const L2PipeKernel* find_l2pipe(int prec, int64_t n, int dir, int n1 = 0, int nc1 = 0, int nc2 = 0, int nst = 0);

@@ -1,0 +1,93 @@
+"""Packed-pair multi-pass kernels (complex64 2^15..2^24) against the FP64 FFT:
+every length, both directions, batches, in place, and buffers
+off 16 bytes, which take the scalar kernels of the same split."""
+import pytest
+
+import algofft
+from helpers import tol_c2c
+
+pytestmark = pytest.mark.gpu
+
+LENGTHS = [1 << k for k in range(15, 25)]
+
+
+def _token(n):
+    return next(t for t in algofft.Variants(n) if t.endswith("-pair"))
+
+
+def _data(n, count, seed):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    return torch.view_as_complex(torch.randn(n * count, 2, generator=g, device="cuda"))
+
+
+def _err(got, want):
+    import torch
+    return float(torch.linalg.vector_norm(got - want) / torch.linalg.vector_norm(want))
+
+
+@pytest.mark.parametrize("n", LENGTHS)
+def test_pair_lengths(n):
+    import torch
+    count = max(1, min(3, (1 << 25) // n))
+    x = _data(n, count, n % 997)
+    ref = torch.fft.fft(x.view(count, n).to(torch.complex128), dim=1).view(-1)
+    y = torch.empty_like(x)
+    with algofft.Plan(n, variant=_token(n)) as p:
+        assert p.Algorithm() == _token(n)
+        p.ForwardBatch(y, x, count)
+        assert _err(y, ref) <= tol_c2c(n, False)
+        b = torch.empty_like(x)
+        p.InverseBatch(b, y, count)
+        assert _err(b, x) <= 2 * tol_c2c(n, False)
+        z = x.clone()
+        p.ForwardBatch(z, z, count)  # in place
+        assert torch.equal(torch.view_as_real(z), torch.view_as_real(y))
+        one = torch.empty_like(x[:n])
+        p.Forward(one, x[:n])
+        assert torch.equal(torch.view_as_real(one), torch.view_as_real(y[:n]))
+
+
+@pytest.mark.parametrize("n", [1 << 15, 1 << 16, 1 << 17, 1 << 18, 1 << 19, 1 << 20, 1 << 21])
+def test_pair_small_and_full_grids_agree(n):
+    # one transform and a batch on either side of the grid-size rule
+    import torch
+    for count in (1, 2, 5, 37):
+        if n * count > 1 << 25:
+            continue
+        x = _data(n, count, count)
+        ref = torch.fft.ifft(x.view(count, n).to(torch.complex128), dim=1).view(-1)
+        y = torch.empty_like(x)
+        with algofft.Plan(n, variant=_token(n)) as p:
+            for _ in range(3):  # launches that follow one another without a wait
+                p.InverseBatch(y, x, count)
+        assert _err(y, ref) <= tol_c2c(n, False)
+
+
+@pytest.mark.parametrize("n", [1 << 15, 1 << 18, 1 << 19, 1 << 21])
+def test_pair_unaligned_buffers(n):
+    import torch
+    x = _data(n + 1, 2, 3)
+    ref = torch.fft.fft(x[1:1 + 2 * n].view(2, n).to(torch.complex128), dim=1).view(-1)
+    d = torch.full((2 * n + 1,), 9 + 0j, dtype=torch.complex64, device="cuda")
+    with algofft.Plan(n, variant=_token(n)) as p:
+        p.ForwardBatch(d[1:], x[1:1 + 2 * n], 2)
+        assert _err(d[1:], ref) <= tol_c2c(n, False)
+        assert complex(d[0].item()) == 9
+        aligned = torch.empty(2 * n, dtype=torch.complex64, device="cuda")
+        p.ForwardBatch(aligned, x[1:1 + 2 * n], 2)  # only the source is off 16 bytes
+        assert _err(aligned, ref) <= tol_c2c(n, False)
+
+
+def test_pair_is_the_default_and_old_tokens_still_run():
+    import torch
+    n = 1 << 16
+    x = _data(n, 2, 5)
+    ref = torch.fft.fft(x.view(2, n).to(torch.complex128), dim=1).view(-1)
+    for tok in [None] + [t for t in algofft.Variants(n) if "-tp-" in t]:
+        y = torch.empty_like(x)
+        with (algofft.Plan(n, variant=tok) if tok else algofft.NewPlan(n)) as p:
+            assert tok or p.Algorithm().endswith("-pair")
+            p.ForwardBatch(y, x, 2)
+        assert _err(y, ref) <= tol_c2c(n, False)
