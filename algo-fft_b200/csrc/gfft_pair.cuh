@@ -169,13 +169,14 @@ __device__ __forceinline__ float4 pair_raw(Pair p) { return float4{p.x.v.x, p.y.
 // columns).
 template <int L, int EPT, int NP>
 struct PairShape {
-  static_assert(NP == 4 || NP == 8 || NP == 16 || NP == 32, "4 to 32 column pairs per tile");
+  static_assert(NP == 2 || NP == 4 || NP == 8 || NP == 16 || NP == 32, "2 to 32 column pairs per tile");
   static constexpr int T = L / EPT;
   static constexpr int TPB = T * NP;
   static constexpr int SMEM = L * NP * 16;
   static constexpr int LE = EPT == 4 ? 2 : EPT == 8 ? 3 : EPT == 16 ? 4 : 5;
   __device__ static __forceinline__ int phys(int row, int c) {
-    if constexpr (NP == 4) return (row ^ ((row >> LE) & 1)) * 4 + (c ^ ((row >> 1) & 3));
+    if constexpr (NP == 2) return (row ^ ((row >> LE) & 3)) * 2 + (c ^ ((row >> 2) & 1));
+    else if constexpr (NP == 4) return (row ^ ((row >> LE) & 1)) * 4 + (c ^ ((row >> 1) & 3));
     else return row * NP + (c ^ (row & 7));
   }
 };

@@ -206,6 +206,34 @@ __device__ __forceinline__ void pair_columns(float4* sh, const float2* __restric
   pair_stage<L, EPT, NP, DIR, 1>(v, sh, threadIdx.x / NP, threadIdx.x % NP, tw, ld, st);
 }
 
+// Rows at a run-time pitch (in pairs; a tile spans less than 2^32 pairs), for
+// tiles whose last pairs may lie beyond the array (active = false).
+template <typename TW>
+struct PairStridedLoad : TW {
+  const float4* in;
+  unsigned pitch;
+  bool active;
+  __device__ __forceinline__ Pair operator()(int row, int c) const {
+    return active ? pair_of(__ldcg(in + (unsigned(row) * pitch + unsigned(c)))) : Pair{V2(0.0), V2(0.0)};
+  }
+};
+template <bool SCALE>
+struct PairStridedStore {
+  static constexpr bool ROWS_FIRST = false;
+  template <int RS, int P, int DIR> using Factors = PairNoFactors;
+  float4* out;
+  unsigned pitch;
+  bool active;
+  float scale;
+  __device__ __forceinline__ void operator()(int row, int c, Pair o) const {
+    if constexpr (SCALE) {
+      const V2 s(float2{scale, scale});
+      o = Pair{o.x * s, o.y * s};
+    }
+    if (active) __stcs(out + (unsigned(row) * pitch + unsigned(c)), pair_raw(o));
+  }
+};
+
 struct PairPassParams {
   const float2* src;
   float2* dst;

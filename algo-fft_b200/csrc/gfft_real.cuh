@@ -57,7 +57,9 @@ k_r2c_pow2(const C* src, C* dst, int64_t count, int64_t idist, int64_t odist, co
   const int t = threadIdx.x % S::T;
   const int64_t b = int64_t(blockIdx.x) * S::B + threadIdx.x / S::T;
   const bool valid = b < count;
-  GlobalLoad<C> ld{src + (valid ? b * idist : 0), valid};
+  // evict-first: the spectrum, not the input, is what a next pass reads from L2
+  // (real 1024 x 1024 arrays x 16: 158 us, 164 with the default)
+  GlobalLoad<C, true> ld{src + (valid ? b * idist : 0), valid};
   PaddedStore<C, H, EPT> st{sh};
   pow2_fft<C, H, EPT, -1>(sh, t, tw, ld, st);
   xsync<S::T>();

@@ -91,3 +91,19 @@ def test_pair_is_the_default_and_old_tokens_still_run():
             assert tok or p.Algorithm().endswith("-pair")
             p.ForwardBatch(y, x, 2)
         assert _err(y, ref) <= tol_c2c(n, False)
+
+
+@pytest.mark.parametrize("L", [32, 64, 128, 256, 512, 1024, 2048, 4096])
+@pytest.mark.parametrize("cols,offset", [(2, 0), (66, 0), (62, 0), (33, 0), (64, 1)])
+def test_pair_columns(L, cols, offset):
+    # column batches: partial tiles, odd pitches and buffers off 16 bytes (the
+    # scalar tile), both directions, out of and in place
+    import torch
+    x = _data(L * cols + offset, 1, L + cols)[offset:]
+    ref = torch.fft.fft(x.view(L, cols).to(torch.complex128), dim=0).reshape(-1)
+    y = torch.empty(L * cols + offset, dtype=torch.complex64, device="cuda")[offset:]
+    with algofft.NewPlan(L) as p:
+        p.StridedBatch(y, x, cols, cols, 1)
+        assert _err(y, ref) <= tol_c2c(L, False)
+        p.StridedBatch(y, y, cols, cols, 1, inverse=True)
+        assert _err(y, x) <= 2 * tol_c2c(L, False)
