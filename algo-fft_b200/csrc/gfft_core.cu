@@ -653,6 +653,19 @@ static bool pair_aligned(const void* dst, const void* src, int64_t idist, int64_
          odist % 2 == 0;
 }
 
+// Whether a two-pass call can keep its intermediate in dst: pass 1 stores Y as
+// N2 rows of N1, and pass 2 transforms the columns of that matrix into the
+// columns of the output, each tile reading its columns before it writes them.
+// It takes contiguous outputs that no input shares memory with.
+bool dst_holds_intermediate(const PlanCore* c, const void* dst, const void* src, int64_t count, int64_t idist,
+                            int64_t odist) {
+  if (odist != c->n || idist < 0) return false;
+  const uintptr_t es = elem_bytes(c->prec), d = reinterpret_cast<uintptr_t>(dst), s = reinterpret_cast<uintptr_t>(src);
+  const uintptr_t din = (uintptr_t(count - 1) * uintptr_t(idist) + uintptr_t(c->n)) * es;
+  const uintptr_t dout = uintptr_t(count) * uintptr_t(c->n) * es;
+  return d + dout <= s || s + din <= d;
+}
+
 // Parameters of the scalar two-pass kernels of a plan.
 static TwoPassParams twopass_params(const PlanCore* c, int dir, void* dst, const void* src, void* ws, int64_t count,
                                     int64_t idist, int64_t odist) {
@@ -681,9 +694,10 @@ static gfft_status exec_pair(const PlanCore* c, int dir, void* dst, const void* 
   const PairKernel* k = c->pair;
   const int d = dir < 0 ? 0 : 1;
   const int64_t tbytes = c->n * int64_t(sizeof(float2)), m1 = c->n / k->n1;
+  const bool own = k->m2 || !dst_holds_intermediate(c, dst, src, count, idist, odist);
   const int64_t nb = std::max<int64_t>(1, std::min<int64_t>(count, (int64_t(1) << 30) / tbytes));
-  void* ws = nullptr;
-  GFFT_CUDA(ws_alloc(&ws, size_t(nb) * size_t(tbytes), st));
+  void* ws = dst;
+  if (own) GFFT_CUDA(ws_alloc(&ws, size_t(nb) * size_t(tbytes), st));
   PairPassParams p{};
   p.scratch = static_cast<float2*>(ws);
   p.idist = idist;
@@ -696,13 +710,13 @@ static gfft_status exec_pair(const PlanCore* c, int dir, void* dst, const void* 
   p.ts = static_cast<const float2*>(c->pair_tw);
   p.ts4 = p.ts + m1;
   p.scale = dir < 0 ? 1.f : float(1.0 / double(c->n));
-  const TwoPassParams sp =
-      k->first_only ? twopass_params(c, dir, dst, src, ws, count, idist, odist) : TwoPassParams{};
+  TwoPassParams sp = k->first_only ? twopass_params(c, dir, dst, src, ws, count, idist, odist) : TwoPassParams{};
   cudaError_t e = cudaSuccess;
   for (int64_t b0 = 0; b0 < count && e == cudaSuccess; b0 += nb) {
     const int64_t m = std::min(nb, count - b0);
     p.src = static_cast<const float2*>(src) + b0 * idist;
     p.dst = static_cast<float2*>(dst) + b0 * odist;
+    if (!own) sp.scratch = p.scratch = p.dst;
     e = k->launch[d](p, 1, m, st);
     if (k->first_only) {
       if (e == cudaSuccess) e = c->tp[d]->split(sp, 2, b0, m, st);
@@ -710,29 +724,32 @@ static gfft_status exec_pair(const PlanCore* c, int dir, void* dst, const void* 
     }
     for (int pass = 2; pass <= (k->m2 ? 3 : 2) && e == cudaSuccess; ++pass) e = k->launch[d](p, pass, m, st);
   }
-  cudaFreeAsync(ws, st);
+  if (own) cudaFreeAsync(ws, st);
   if (e != cudaSuccess) return cuda_status(e, "k_pair");
   return GFFT_OK;
 }
 
 // Two-pass execution in the split schedule (k_tp_split): per chunk of up to
 // 1 GiB of intermediate, one pass-1 launch and one pass-2 launch.  The
-// scratch comes from the library's workspace pool.
+// intermediate lives in dst where it can, else in scratch from the library's
+// workspace pool.
 static gfft_status exec_twopass(const PlanCore* c, int dir, void* dst, const void* src, int64_t count,
                                 int64_t idist, int64_t odist, cudaStream_t st) {
   const TwoPassKernel* k = c->tp[dir < 0 ? 0 : 1];
   const int64_t tbytes = c->n * int64_t(elem_bytes(c->prec));
   const int64_t nb = std::max<int64_t>(1, std::min<int64_t>(count, (int64_t(1) << 30) / tbytes));
-  void* ws = nullptr;
-  GFFT_CUDA(ws_alloc(reinterpret_cast<void**>(&ws), size_t(nb) * size_t(tbytes), st));
-  const TwoPassParams p = twopass_params(c, dir, dst, src, ws, count, idist, odist);
+  const bool own = !dst_holds_intermediate(c, dst, src, count, idist, odist);
+  void* ws = dst;
+  if (own) GFFT_CUDA(ws_alloc(reinterpret_cast<void**>(&ws), size_t(nb) * size_t(tbytes), st));
+  TwoPassParams p = twopass_params(c, dir, dst, src, ws, count, idist, odist);
   cudaError_t e = cudaSuccess;
   for (int64_t b0 = 0; b0 < count && e == cudaSuccess; b0 += nb) {
     const int64_t m = std::min(nb, count - b0);
+    if (!own) p.scratch = static_cast<char*>(dst) + b0 * tbytes;
     e = k->split(p, 1, b0, m, st);
     if (e == cudaSuccess) e = k->split(p, 2, b0, m, st);
   }
-  cudaFreeAsync(ws, st);
+  if (own) cudaFreeAsync(ws, st);
   if (e != cudaSuccess) return cuda_status(e, "k_tp_split");
   return GFFT_OK;
 }

@@ -212,6 +212,9 @@ cudaError_t exec_bluestein_fused(int prec, int64_t M, const void* src, void* dst
 gfft_status exec_runtime_plan(const PlanCore* c, int dir, void* dst, const void* src, int64_t count, int64_t idist,
                               int64_t odist, cudaStream_t st);
 
+bool dst_holds_intermediate(const PlanCore* c, const void* dst, const void* src, int64_t count, int64_t idist,
+                            int64_t odist);
+
 // Fills dst[j] = W_n^{(j*step) mod n} for j < count (FP64, rounded).
 // Stream-ordered workspace from the library's per-device pool (released
 // with cudaFreeAsync; the pool keeps the memory for later calls).

@@ -301,8 +301,9 @@ static gfft_status exec_gen_twopass(const PlanCore* c, int dir, void* dst, const
   const size_t es = elem_bytes(c->prec);
   const int64_t n = c->n;
   const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(count, (int64_t(512) << 20) / (n * int64_t(es))));
+  const bool own = !dst_holds_intermediate(c, dst, src, count, idist, odist);
   void* scratch = nullptr;
-  GFFT_CUDA(ws_alloc(reinterpret_cast<void**>(&scratch), size_t(chunk) * size_t(n) * es, st));
+  if (own) GFFT_CUDA(ws_alloc(reinterpret_cast<void**>(&scratch), size_t(chunk) * size_t(n) * es, st));
   BigTwiddle bt{c->bt_lo, c->bt_hi, c->bt_shift};
   const double scale = 1.0 / double(n);
   cudaError_t e = cudaSuccess;
@@ -310,6 +311,7 @@ static gfft_status exec_gen_twopass(const PlanCore* c, int dir, void* dst, const
     const int64_t m = std::min(chunk, count - b0);
     const char* in = static_cast<const char*>(src) + size_t(b0) * size_t(idist) * es;
     char* out = static_cast<char*>(dst) + size_t(b0) * size_t(odist) * es;
+    if (!own) scratch = out;
     if (c->mixc) {
       e = mixc_passes(c, dir, in, scratch, out, m, idist, odist, bt, scale, st);
     } else if (c->prec == kC64) {
@@ -322,7 +324,7 @@ static gfft_status exec_gen_twopass(const PlanCore* c, int dir, void* dst, const
         e = launch_cols<double2, GEN_PASS2>(c->gs2, dir, scratch, out, m, n, odist, c->gn1, c->tw2, bt, scale, st);
     }
   }
-  cudaFreeAsync(scratch, st);
+  if (own) cudaFreeAsync(scratch, st);
   if (e != cudaSuccess) return cuda_status(e, c->mixc ? "k_mix_cols" : "k_gen_cols");
   return GFFT_OK;
 }

@@ -107,3 +107,23 @@ def test_pair_columns(L, cols, offset):
         assert _err(y, ref) <= tol_c2c(L, False)
         p.StridedBatch(y, y, cols, cols, 1, inverse=True)
         assert _err(y, x) <= 2 * tol_c2c(L, False)
+
+
+@pytest.mark.parametrize("n,prec", [(1 << 15, 0), (1 << 18, 0), (1 << 20, 0), (1 << 16, 1), (50421, 0), (100000, 1),
+                                    (1 << 21, 1)])
+@pytest.mark.parametrize("shift", [0, 2, None])
+def test_two_pass_outputs_that_overlap_their_inputs(n, prec, shift):
+    # the intermediate lives in dst unless dst shares memory with src (the same
+    # buffer, or one that starts a little later); None: separate buffers
+    import torch
+    count, dt = 3, (torch.complex128 if prec else torch.complex64)
+    x = _data(n, count, 11).to(dt)
+    ref = torch.fft.fft(x.view(count, n).to(torch.complex128), dim=1).view(-1)
+    buf = torch.empty(n * count + 8, dtype=dt, device="cuda")
+    src = buf[:n * count] if shift is not None else x
+    if shift is not None:
+        src.copy_(x)
+    dst = buf[shift or 0:(shift or 0) + n * count]
+    with algofft.NewPlanT(n, prec) as p:
+        p.ForwardBatch(dst, src, count)
+    assert _err(dst, ref) <= tol_c2c(n, bool(prec))
