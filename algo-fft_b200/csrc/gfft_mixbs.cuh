@@ -124,6 +124,8 @@ struct MixBsOut {
 // transform * tiles + tile; item mode: items[blk[blockIdx]]).
 template <typename C, typename SC, int NC, int KIND, int MINB = 1, int TT = 0>
 __global__ void __launch_bounds__(MixTile<SC, NC, TT>::TPB, MINB) k_mix_bs(MixBsParams p) {
+  if constexpr (KIND != BSK_OUT) asm volatile("griddepcontrol.launch_dependents;");
+  if constexpr (KIND != BSK_IN) asm volatile("griddepcontrol.wait;" ::: "memory");  // the pass before this one
   using TL = MixTile<SC, NC, TT>;
   using Re = typename RealOf<C>::type;
   constexpr int L = SC::L;

@@ -79,7 +79,29 @@ __device__ __forceinline__ void ptwiddle_block(Pair* a) {
   }
 }
 
-// In-register DFT of R pairs (R a power of two up to 32), natural order.
+// Odd prime radix (3, 5, 7): dft_odd on pairs.
+template <int R, int K, int J>
+__device__ __forceinline__ void podd_accum(Pair& a, Pair& b, const Pair* s, const Pair* d) {
+  if constexpr (J <= (R - 1) / 2) {
+    const V2 c(cos_r<R>((J * K) % R)), sn(sin_r<R>((J * K) % R));
+    a = Pair{fma2(s[J].x, c, a.x), fma2(s[J].y, c, a.y)};
+    if constexpr (J == 1) b = Pair{d[J].x * sn, d[J].y * sn};
+    else b = Pair{fma2(d[J].x, sn, b.x), fma2(d[J].y, sn, b.y)};
+    podd_accum<R, K, J + 1>(a, b, s, d);
+  }
+}
+template <int R, int K, int DIR>
+__device__ __forceinline__ void podd_out(Pair* v, const Pair* s, const Pair* d, Pair x0) {
+  if constexpr (K <= (R - 1) / 2) {
+    Pair a = x0, b;
+    podd_accum<R, K, 1>(a, b, s, d);
+    v[K] = padd_i<DIR>(a, b);
+    v[R - K] = padd_i<-DIR>(a, b);
+    podd_out<R, K + 1, DIR>(v, s, d, x0);
+  }
+}
+
+// In-register DFT of R pairs (7-smooth R up to 64), natural order.
 template <int R, int DIR>
 __device__ __forceinline__ void pdft(Pair* v) {
   if constexpr (R == 1) {
@@ -94,6 +116,20 @@ __device__ __forceinline__ void pdft(Pair* v) {
     v[2] = csub(t0, t2);
     v[1] = padd_i<DIR>(t1, d);
     v[3] = padd_i<-DIR>(t1, d);
+  } else if constexpr (R == 3 || R == 5 || R == 7) {
+    constexpr int H = (R - 1) / 2;
+    Pair s[H + 1], d[H + 1];
+#pragma unroll
+    for (int j = 1; j <= H; ++j) {
+      s[j] = cadd(v[j], v[R - j]);
+      d[j] = csub(v[j], v[R - j]);
+    }
+    const Pair x0 = v[0];
+    Pair sum = x0;
+#pragma unroll
+    for (int j = 1; j <= H; ++j) sum = cadd(sum, s[j]);
+    podd_out<R, 1, DIR>(v, s, d, x0);
+    v[0] = sum;
   } else {
     constexpr int R1 = dft_split(R), R2 = R / R1;
     Pair a[R];
@@ -119,7 +155,7 @@ __device__ __forceinline__ void pdft(Pair* v) {
   }
 }
 
-// Powers w^r, r < RS <= 32, of one factor per thread from exactly rounded
+// Powers w^r, r < RS <= 64, of one factor per thread from exactly rounded
 // table entries: lo[1], lo[2], lo[4] and hi[h] = w^(8h) are loaded, the others
 // are products of two (w^r = lo[r mod 8] hi[r / 8]).  A tree that starts from
 // w alone multiplies its rounding error by r.

@@ -438,14 +438,15 @@ gfft_status init_bluestein(PlanCore* c, int mode) {
   const int64_t nlo = int64_t(1) << shift, nhi = (M + nlo - 1) >> shift;
   const int64_t m2 = bsm ? M / m1 : 0;
   const int64_t extra = bsm ? m1 + m2 + nlo + nhi : 0;
-  GFFT_CUDA(cudaMalloc(&c->tw, size_t(2 * n + 2 * M + extra) * es));
+  const int64_t np = (n + 1) & ~int64_t(1);  // every table on 16 bytes (k_mix_bs_pair)
+  GFFT_CUDA(cudaMalloc(&c->tw, size_t(2 * np + 2 * M + extra) * es));
   char* base = static_cast<char*>(c->tw);
   void* wf = base;
-  void* wi = base + n * es;
-  void* ff = base + 2 * n * es;
-  void* fi = base + (2 * n + M) * es;
+  void* wi = base + np * es;
+  void* ff = base + 2 * np * es;
+  void* fi = base + (2 * np + M) * es;
   if (bsm) {
-    char* t = base + (2 * n + 2 * M) * es;
+    char* t = base + (2 * np + 2 * M) * es;
     s = fill_twiddles(c->prec, t, m1, m1, 1, 0);
     if (s == GFFT_OK) s = fill_twiddles(c->prec, t + m1 * es, m2, m2, 1, 0);
     if (s == GFFT_OK) s = fill_twiddles(c->prec, t + (m1 + m2) * es, M, nlo, 1, 0);

@@ -7,6 +7,7 @@
 #include "gfft_internal.h"
 #include "gfft_mixbs.cuh"
 #include "gfft_mixcols.cuh"
+#include "gfft_mixpair.cuh"
 
 namespace gfft {
 
@@ -76,6 +77,26 @@ struct MixBsEntry {
   MixBsFn fn[2][3];    // [prec][BSK_IN / BSK_MID / BSK_OUT]
 };
 
+// In batch mode the middle and last passes launch while the pass before them
+// drains (they wait for it before they read): one call of one transform is
+// three short launches.
+inline cudaError_t launch_mix_bs_kernel(void (*kern)(MixBsParams), const MixBsParams& p, int kind, int64_t blocks,
+                                        int tpb, int smem, cudaStream_t st) {
+  if (blocks <= 0) return cudaSuccess;
+  if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(blocks));
+  cfg.blockDim = dim3(tpb);
+  cfg.dynamicSmemBytes = size_t(smem);
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = kind != BSK_IN && !p.items ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, p);
+}
+
 template <typename C, typename CFG, int KIND>
 cudaError_t launch_mix_bs(const MixBsParams& p, int64_t blocks, cudaStream_t st) {
   using SC = typename CFG::Sched;
@@ -86,10 +107,42 @@ cudaError_t launch_mix_bs(const MixBsParams& p, int64_t blocks, cudaStream_t st)
   static const cudaError_t attr =
       smem > 48 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) : cudaSuccess;
   if (attr != cudaSuccess) return attr;
-  if (blocks <= 0) return cudaSuccess;
-  if (blocks > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
-  kern<<<unsigned(blocks), TL::TPB, smem, st>>>(p);
-  return cudaGetLastError();
+  return launch_mix_bs_kernel(kern, p, KIND, blocks, TL::TPB, smem, st);
+}
+
+// Whether a complex64 pass of the chain runs on packed pairs: tiles of 16
+// columns; the middle pass where its transposed runs of T elements are whole
+// 128-byte lines (16 x 15: 100 -> 91 us, 16 x 16: 91 -> 82, against 94 -> 113 for
+// 16 x 10 with T = 10) and a thread holds at most 20 pairs (21 x 16 lost 3 % of
+// the whole chain), the last pass from 12 threads per column (12 x 12: 52 -> 46
+// us, 14 x 8: 54 -> 52, 16 x 10: 57 -> 58).
+template <typename CFG, int KIND>
+constexpr bool mix_bs_paired() {
+  using SC = typename CFG::Sched;
+  constexpr int T = CFG::tt > 0 ? CFG::tt : SC::L / SC::rmax();
+  constexpr int V = MixPairTile<SC, CFG::tt>::vmax();
+  if (CFG::nc != 2 * kMixPairs || SC::NS != 2) return false;
+  return KIND == BSK_MID ? T % 16 == 0 && V <= 20 : KIND == BSK_OUT && (T >= 12 || T == 8) && V <= 24;
+}
+
+template <typename CFG, int KIND>
+cudaError_t launch_mix_bs_pair(const MixBsParams& p, int64_t blocks, cudaStream_t st) {
+  using TL = MixPairTile<typename CFG::Sched, CFG::tt>;
+  if constexpr (TL::SMEM > 48 * 1024) {
+    const cudaError_t e = raise_smem<&k_mix_bs_pair<typename CFG::Sched, KIND, CFG::tt>>(TL::SMEM);
+    if (e != cudaSuccess) return e;
+  }
+  return launch_mix_bs_kernel(&k_mix_bs_pair<typename CFG::Sched, KIND, CFG::tt>, p, KIND, blocks, TL::TPB, TL::SMEM,
+                              st);
+}
+
+// Uneven batches launch one grid per column length; on a small one (fewer than
+// two CTAs per SM) the scalar tiles' twice as many threads are faster (300
+// transforms: 323 us, 328 in pairs; 4000: 1430 and 1409).
+template <typename CFG, int KIND>
+cudaError_t launch_mix_bs_either(const MixBsParams& p, int64_t blocks, cudaStream_t st) {
+  if (p.items && blocks < 2 * 148) return launch_mix_bs<float2, CFG, KIND>(p, blocks, st);
+  return launch_mix_bs_pair<CFG, KIND>(p, blocks, st);
 }
 
 // Bluestein-chain entry of length L from its complex64 and complex128
@@ -102,8 +155,10 @@ MixBsEntry mix_bs_entry() {
   e.nc[kC64] = F::nc;
   e.nc[kC128] = D::nc;
   e.fn[kC64][BSK_IN] = &launch_mix_bs<float2, F, BSK_IN>;
-  e.fn[kC64][BSK_MID] = &launch_mix_bs<float2, F, BSK_MID>;
-  e.fn[kC64][BSK_OUT] = &launch_mix_bs<float2, F, BSK_OUT>;
+  if constexpr (mix_bs_paired<F, BSK_MID>()) e.fn[kC64][BSK_MID] = &launch_mix_bs_either<F, BSK_MID>;
+  else e.fn[kC64][BSK_MID] = &launch_mix_bs<float2, F, BSK_MID>;
+  if constexpr (mix_bs_paired<F, BSK_OUT>()) e.fn[kC64][BSK_OUT] = &launch_mix_bs_either<F, BSK_OUT>;
+  else e.fn[kC64][BSK_OUT] = &launch_mix_bs<float2, F, BSK_OUT>;
   e.fn[kC128][BSK_IN] = &launch_mix_bs<double2, D, BSK_IN>;
   e.fn[kC128][BSK_MID] = &launch_mix_bs<double2, D, BSK_MID>;
   e.fn[kC128][BSK_OUT] = &launch_mix_bs<double2, D, BSK_OUT>;

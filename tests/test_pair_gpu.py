@@ -127,3 +127,22 @@ def test_two_pass_outputs_that_overlap_their_inputs(n, prec, shift):
     with algofft.NewPlanT(n, prec) as p:
         p.ForwardBatch(dst, src, count)
     assert _err(dst, ref) <= tol_c2c(n, bool(prec))
+
+
+@pytest.mark.parametrize("n", [9437, 13007, 16411, 27793, 33013])
+@pytest.mark.parametrize("count", [1, 7])
+def test_bluestein_pair_passes(n, count):
+    # M = 80 x 240, 112 x 240, 144 x 240, 224 x 256, 240 x 288: middle and last
+    # passes in pairs or scalar by length; odd n puts every other transform off
+    # 16 bytes, and the last pair of an odd n is half there
+    import torch
+    x = _data(n, count, n)
+    ref = torch.fft.fft(x.view(count, n).to(torch.complex128), dim=1).view(-1)
+    guard = torch.full((n * count + 2,), 5 + 0j, dtype=torch.complex64, device="cuda")
+    y = guard[:n * count]
+    with algofft.NewPlan(n) as p:
+        p.ForwardBatch(y, x, count)
+        assert _err(y, ref) <= tol_c2c(4 * n, False)
+        assert (guard[n * count:] == 5).all()
+        p.InverseBatch(y, y, count)
+        assert _err(y, x) <= 2 * tol_c2c(4 * n, False)
