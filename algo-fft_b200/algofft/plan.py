@@ -44,26 +44,42 @@ def _ptr_len(x):
     if _is_device(x):
         if not x.is_contiguous():
             raise ValueError("device tensors must be contiguous")
-        return ctypes.c_void_p(x.data_ptr()), x.numel(), True
+        return x.data_ptr(), x.numel(), True
     if isinstance(x, np.ndarray):
         if not x.flags.c_contiguous:
             raise ValueError("host arrays must be C-contiguous")
-        return ctypes.c_void_p(x.ctypes.data), x.size, False
+        return x.ctypes.data, x.size, False
     raise TypeError(f"unsupported buffer type {type(x)}")
 
 
+_raw_stream = None  # device index -> handle of torch's current stream
+
+
 def _stream(x):
-    import torch
-    return ctypes.c_void_p(torch.cuda.current_stream(x.device).cuda_stream)
+    """Handle of torch's current stream on the tensor's device."""
+    global _raw_stream
+    if _raw_stream is None:
+        import torch
+        _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+            lambda i: torch.cuda.current_stream(i).cuda_stream)
+    return _raw_stream(x.get_device())
+
+
+_precs: dict = {}  # element type -> precision
 
 
 def _dtype_prec(dtype) -> int:
-    s = str(dtype)
-    if s.endswith("complex64"):
-        return COMPLEX64
-    if s.endswith("complex128"):
-        return COMPLEX128
-    raise TypeError(f"unsupported element type {dtype}")
+    p = _precs.get(dtype)
+    if p is None:
+        s = str(dtype)
+        if s.endswith("complex64"):
+            p = COMPLEX64
+        elif s.endswith("complex128"):
+            p = COMPLEX128
+        else:
+            raise TypeError(f"unsupported element type {dtype}")
+        _precs[dtype] = p
+    return p
 
 
 class Plan:
