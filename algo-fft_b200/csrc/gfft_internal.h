@@ -149,7 +149,8 @@ struct MixBsParams;
 struct MixRowsParams;
 bool mix_rows_supported(int prec, int64_t L);
 cudaError_t exec_mix_rows(int prec, int dir, int64_t L, const MixRowsParams& p, cudaStream_t st);
-int64_t bs_mixed_length(int64_t n, int64_t* m1);
+// (the length M does not depend on the precision, its split M1 x M2 does)
+int64_t bs_mixed_length(int64_t n, int64_t* m1, int prec = kC64);
 int mix_bs_width(int prec, int64_t L);
 cudaError_t exec_mix_bs(int prec, int kind, int64_t L, MixBsParams p, int64_t count, cudaStream_t st);
 // Bluestein's FFT length: kBsAuto takes the mixed length (a product of
@@ -158,7 +159,7 @@ cudaError_t exec_mix_bs(int prec, int kind, int64_t L, MixBsParams p, int64_t co
 // latter where a smaller mixed length exists).  bs_mixed_choice: that
 // smaller mixed length (0: none, or the one-CTA fused range).
 enum { kBsAuto = 0, kBsPow2 = 1, kBsMixed = 2 };
-int64_t bs_mixed_choice(int64_t n, int64_t* m1);
+int64_t bs_mixed_choice(int64_t n, int64_t* m1, int prec = kC64);
 bool bs_mixed_preferred(int64_t mx, int64_t M);
 gfft_status init_bluestein(PlanCore* c, int mode = kBsAuto);
 // Tensor-core split-fp16 radix-16 form (complex64, powers of two 16 <= n <= 2^24;

@@ -389,10 +389,10 @@ __global__ void k_bs_post(C* y, const C* work, const C* w, int64_t n, int64_t M,
 
 static unsigned grid_for(int64_t total) { return unsigned(std::max<int64_t>(1, std::min<int64_t>((total + 255) / 256, 148 * 32))); }
 
-int64_t bs_mixed_choice(int64_t n, int64_t* m1) {
+int64_t bs_mixed_choice(int64_t n, int64_t* m1, int prec) {
   int64_t M = 1;
   while (M < 2 * n - 1) M <<= 1;
-  const int64_t mx = bs_mixed_length(n, m1);
+  const int64_t mx = bs_mixed_length(n, m1, prec);
   return M > 16384 && mx > 0 && mx < M ? mx : 0;
 }
 
@@ -415,7 +415,7 @@ gfft_status init_bluestein(PlanCore* c, int mode) {
   // compiled column lengths (the product is the same up to rounding) where
   // bs_mixed_preferred expects it to be faster.
   int64_t m1 = 0;
-  const int64_t mx = bs_mixed_choice(n, &m1);
+  const int64_t mx = bs_mixed_choice(n, &m1, c->prec);
   const bool bsm = mx > 0 && (mode == kBsMixed || (mode == kBsAuto && bs_mixed_preferred(mx, M)));
   if (bsm) M = mx;
   const size_t es = elem_bytes(c->prec);

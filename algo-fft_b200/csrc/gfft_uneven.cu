@@ -238,7 +238,7 @@ static gfft_status uneven_build(gfft_plan_uneven* p) {
     // column lengths where the plans' rule prefers it (never a power of
     // two itself)
     int64_t bm1 = 0;
-    const int64_t mx = M > max_direct_bs ? bs_mixed_choice(n, &bm1) : 0;
+    const int64_t mx = M > max_direct_bs ? bs_mixed_choice(n, &bm1, p->prec) : 0;
     if (bs_mixed_preferred(mx, M)) {
       bsm_M[n] = mx;
       bsm_m1[n] = bm1;

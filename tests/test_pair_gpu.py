@@ -129,6 +129,21 @@ def test_two_pass_outputs_that_overlap_their_inputs(n, prec, shift):
     assert _err(dst, ref) <= tol_c2c(n, bool(prec))
 
 
+@pytest.mark.parametrize("n", [50789, 52433, 58963, 40993])
+@pytest.mark.parametrize("prec", [0, 1])
+def test_bluestein_splits_of_equal_lengths(n, prec):
+    # M = 102400, 107520, 122880, 82944: 256 x 400, 240 x 448, 256 x 480, 192 x 432
+    # (complex128 288 x 288), not the most balanced factors
+    import torch
+    dt = torch.complex128 if prec else torch.complex64
+    x = _data(n, 2, n).to(dt)
+    ref = torch.fft.ifft(x.view(2, n).to(torch.complex128), dim=1).view(-1)
+    y = torch.empty_like(x)
+    with algofft.Plan(n, prec, variant=f"gpu-sm100-bluestein-n{n}-mx") as p:
+        p.InverseBatch(y, x, 2)
+    assert _err(y, ref) <= tol_c2c(4 * n, bool(prec))
+
+
 @pytest.mark.parametrize("n", [9437, 13007, 16411, 27793, 33013])
 @pytest.mark.parametrize("count", [1, 7])
 def test_bluestein_pair_passes(n, count):
