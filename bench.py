@@ -52,7 +52,13 @@ TRAFFIC_PER_TRANSFORM = {"gpu-sm100-tp-4096x4096-t16384-e16": 490.6e6,
                          "gpu-sm100-tp-1024x1024-t8192-e16": 30.77e6,
                          "gpu-sm100-tp-1024x2048-t8192-e16": 61.69e6,
                          "gpu-sm100-tp3t-256x128x128-t4096-e16-s3": 179.92e6,
-                         "gpu-sm100-tp3-256x256x256": 715.25e6}
+                         "gpu-sm100-tp3-256x256x256": 715.25e6,
+                         "gpu-sm100-tp-512x512-t8192-e32-pair": 7.48e6,
+                         "gpu-sm100-tp-1024x1024-t8192-e16-pair": 30.08e6,
+                         "gpu-sm100-tp3-128x128x128-pair": 89.8e6,
+                         "gpu-sm100-tp3-256x128x128-pair": 179.0e6,
+                         "gpu-sm100-tp3-256x256x128-pair": 359.1e6,
+                         "gpu-sm100-tp3-256x256x256-pair": 718.5e6}
 
 
 def launches_of(algorithm: str, count: int, n: int, es: int) -> int:
@@ -854,7 +860,9 @@ def main():
     dom_bytes = bytes_per_transform(dom) * bufs[dom][2] / dom_launches  # algorithmic bytes per launch
     peak, peak_kind = peak_hbm()
     achieved = dom_bytes / (dom_ms / 1e3) / 1e9
-    if "-tp3t-" in dom_alg:
+    if dom_alg.endswith("-pair"):
+        kname = f"k_pair_tp (packed column pairs, one launch per pass; N={dom}, {dom_alg})"
+    elif "-tp3t-" in dom_alg:
         kname = f"k_tp3t (TMA-staged three passes, one persistent launch each; N={dom}, {dom_alg})"
     elif "-tp3-" in dom_alg:
         kname = f"k_tp3 (three passes, one launch each; N={dom}, {dom_alg})"
