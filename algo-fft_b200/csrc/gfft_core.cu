@@ -110,6 +110,8 @@ cudaError_t prepare_kernels() {
   if (e != cudaSuccess) return e;
   std::lock_guard<std::mutex> g(mu);
   if (std::find(done.begin(), done.end(), dev) != done.end()) return cudaSuccess;
+  e = ws_prepare();
+  if (e != cudaSuccess) return e;
   for (const auto& k : pow2_table()) {
     if (k.smem > 48 * 1024) {
       e = cudaFuncSetAttribute(k.func, cudaFuncAttributeMaxDynamicSharedMemorySize, k.smem);
@@ -182,31 +184,44 @@ gfft_status make_twiddles(int prec, int64_t n, void** out, cudaStream_t st) {
 // staging) comes from one stream-ordered pool per device that keeps freed
 // memory (release threshold = max): the device's default pool returns its
 // memory at every synchronize, so each call would map its workspace anew.
-cudaError_t ws_alloc(void** p, size_t bytes, cudaStream_t st) {
+static cudaError_t ws_pool(cudaMemPool_t* out) {
   static std::mutex mu;
   static std::vector<std::pair<int, cudaMemPool_t>> pools;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  cudaMemPool_t pool = nullptr;
-  {
-    std::lock_guard<std::mutex> g(mu);
-    for (auto& kv : pools)
-      if (kv.first == dev) pool = kv.second;
-    if (!pool) {
-      cudaMemPoolProps props = {};
-      props.allocType = cudaMemAllocationTypePinned;
-      props.location.type = cudaMemLocationTypeDevice;
-      props.location.id = dev;
-      e = cudaMemPoolCreate(&pool, &props);
-      if (e != cudaSuccess) return e;
-      uint64_t keep = ~uint64_t(0);
-      e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-      if (e != cudaSuccess) return e;
-      pools.emplace_back(dev, pool);
+  std::lock_guard<std::mutex> g(mu);
+  for (auto& kv : pools)
+    if (kv.first == dev) {
+      *out = kv.second;
+      return cudaSuccess;
     }
-  }
-  return cudaMallocFromPoolAsync(p, bytes, pool, st);
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool = nullptr;
+  e = cudaMemPoolCreate(&pool, &props);
+  if (e != cudaSuccess) return e;
+  uint64_t keep = ~uint64_t(0);
+  e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  if (e != cudaSuccess) return e;
+  pools.emplace_back(dev, pool);
+  *out = pool;
+  return cudaSuccess;
+}
+
+// A pool cannot be created while a stream is captured, so plans create their
+// device's before any call of theirs can be.
+cudaError_t ws_prepare() {
+  cudaMemPool_t pool = nullptr;
+  return ws_pool(&pool);
+}
+
+cudaError_t ws_alloc(void** p, size_t bytes, cudaStream_t st) {
+  cudaMemPool_t pool = nullptr;
+  const cudaError_t e = ws_pool(&pool);
+  return e != cudaSuccess ? e : cudaMallocFromPoolAsync(p, bytes, pool, st);
 }
 
 // ---------------------------------------------------------------- copy kernel

@@ -220,6 +220,7 @@ bool dst_holds_intermediate(const PlanCore* c, const void* dst, const void* src,
 // Stream-ordered workspace from the library's per-device pool (released
 // with cudaFreeAsync; the pool keeps the memory for later calls).
 cudaError_t ws_alloc(void** p, size_t bytes, cudaStream_t st);
+cudaError_t ws_prepare();  // creates the current device's pool
 gfft_status fill_twiddles(int prec, void* dst, int64_t n, int64_t count, int64_t step, cudaStream_t st);
 
 // What plan creation knows about the calls a plan will serve; the learned

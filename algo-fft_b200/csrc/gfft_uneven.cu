@@ -176,6 +176,7 @@ extern "C" GFFT_API void gfft_plan_uneven_close(gfft_plan_uneven* p);
 namespace gfft {
 
 static gfft_status uneven_build(gfft_plan_uneven* p) {
+  GFFT_CUDA(ws_prepare());
   const size_t es = elem_bytes(p->prec);
   const int64_t max_direct_bs = p->prec == kC64 ? 16384 : 8192;
   // distinct lengths and their handling

@@ -161,3 +161,26 @@ def test_bluestein_pair_passes(n, count):
         assert (guard[n * count:] == 5).all()
         p.InverseBatch(y, y, count)
         assert _err(y, x) <= 2 * tol_c2c(4 * n, False)
+
+
+@pytest.mark.parametrize("what", ["uneven", "in_place", "three_pass"])
+def test_first_call_of_a_process_can_be_captured(what):
+    # a fresh process whose first workspace is needed inside a stream capture
+    import os
+    import subprocess
+    import sys
+    body = {
+        "uneven": "p = algofft.PlanUneven([65536, 16411, 40013, 1000]); x = c(p.Total()); y = torch.empty_like(x)\n"
+                  "p.Forward(y, x)",
+        "in_place": "p = algofft.NewPlan(1 << 16); y = c(1 << 16); run(lambda: p.Forward(y, y))",
+        "three_pass": "p = algofft.NewPlan(1 << 21); x = c(1 << 21); y = torch.empty_like(x)\n"
+                      "run(lambda: p.Forward(y, x))",
+    }[what]
+    code = ("import sys; sys.path.insert(0, 'algo-fft_b200')\nimport torch, algofft\n"
+            "c = lambda n: torch.ones(n, dtype=torch.complex64, device='cuda')\n"
+            "def run(f):\n    g = torch.cuda.CUDAGraph()\n    s = torch.cuda.Stream()\n"
+            "    with torch.cuda.graph(g, stream=s):\n        f()\n    g.replay()\n"
+            + body + "\ntorch.cuda.synchronize()\nassert abs(y[0].item()) > 1\n")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
