@@ -3,6 +3,7 @@
 // (gfft_mixbs.cuh): the tables the generated kernels_mixcols_t*.cu and
 // kernels_mixbs_t*.cu files fill, and the launchers the plans call.
 #include <algorithm>
+#include "gfft_bssplit.h"
 #include "kernels_mixcols.cuh"
 
 namespace gfft {
@@ -86,28 +87,14 @@ const MixBsEntry* bs_find(int64_t L) {
 bool mix_cols_supported(int64_t L) { return find(L) != nullptr; }
 
 int64_t bs_mixed_length(int64_t n, int64_t* m1, int prec) {
-  int64_t best = 0, a_best = 0;
-  const std::vector<MixBsEntry>& t = bs_table();
-  // M1 is the column length of two passes, M2 that of one, and columns beyond
-  // `wide` rows run at one or two CTAs per SM.  Balanced -> this split: n =
-  // 40993 (M = 82944: 288 x 288 -> 192 x 432) 513 -> 450 us per 2^24 elements,
-  // 50789 (102400: 320 x 320 -> 256 x 400) 576 -> 396; complex128 40993 457 us
-  // balanced, 479 as 192 x 432.
-  const int64_t wide = prec == kC64 ? 256 : 288;
-  for (size_t i = 0; i < t.size(); ++i)
-    for (size_t j = i; j < t.size(); ++j) {
-      const int64_t a = t[i].L, b = t[j].L, m = a * b;
-      if (m < 2 * n - 1) continue;
-      // the smallest M; among equal ones the most balanced split with
-      // M1 <= wide, else the most balanced
-      const bool better = (a <= wide) != (a_best <= wide) ? a <= wide : a > a_best;
-      if (best == 0 || m < best || (m == best && better)) {
-        best = m;
-        a_best = a;
-      }
-    }
-  if (m1) *m1 = a_best;
-  return best;
+  static const std::vector<int64_t> lengths = [] {
+    std::vector<int64_t> v;
+    for (const MixBsEntry& e : bs_table()) v.push_back(e.L);
+    return v;
+  }();
+  const BsSplit s = bs_split(lengths, n, bs_split_wide(prec == kC128));
+  if (m1) *m1 = s.m1;
+  return s.m;
 }
 
 bool mix_rows_supported(int prec, int64_t L) {
