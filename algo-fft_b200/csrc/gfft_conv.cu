@@ -253,17 +253,18 @@ cudaError_t dispatch_conv_os(int64_t L, const double* a, double* dst, int64_t na
 // Against the half-length form it replaced (recombination of bins k and H - k
 // through shared memory, five table loads per bin) this costs four exchanges
 // through shared memory instead of seven and two table loads per bin pair.
-// The two blocks are neighbours in one signal: their rounding errors mix only
-// with each other's, and no value crosses between signals.
+// The two blocks are neighbours in one signal: non-finite values and rounding
+// errors reach both blocks and no further, and no value crosses between signals.
 //
 // Bound: the FMA pipe and the phases of one or a few CTAs per SM.  64 signals
 // of 2^20 with 4097 taps: 0.440 ms before (2^15-sample half-length blocks),
-// 0.291 ms now (N = 16384; FMA pipe busy 43 %), rel-L2 error 7.6e-7 -> 3.1e-7;
-// 32 x 2^20 with 513 taps 0.165 -> 0.094 ms (N = 4096; FMA pipe busy 62 %),
-// one signal of 2^17 with 2049 taps 27.9 -> 12.7 us.
+// 0.290 ms now (N = 16384; FMA pipe busy 43 %), rel-L2 error 7.6e-7 -> 3.1e-7;
+// 32 x 2^20 with 513 taps 0.165 -> 0.098 ms, with 33 taps 0.152 -> 0.080 (N =
+// 2048), with 1025 taps 0.169 -> 0.107 (N = 4096).
 using ConvRow16k = PairRow<16384, 32, 16, 16>;
 using ConvRow8k = PairRow<8192, 16, 16, 16>;
 using ConvRow4k = PairRow<4096, 16, 16, 8>;
+using ConvRow2k = PairRow<2048, 16, 8, 8>;
 
 // e in [lo, hi) of a window is a sample of the signal, else zero
 struct PairWindowLoad {
@@ -368,24 +369,30 @@ cudaError_t launch_conv_pair(const float* a, float* dst, int64_t na, int64_t a_d
                             static_cast<const float4*>(hs), PREFETCH && count * npair > resident ? int(resident) : 0);
 }
 
-// Transform length of the float32 blocks: the one whose waves of CTAs take the
-// least time.  `us` is one full wave (148 SMs x resident CTAs), measured on 64
-// signals of 2^20 (513 taps: 4096 points 0.171, 8192 0.205, 16384 0.261 ms;
-// 4097 taps: 8192 points 0.349, 16384 0.306 ms); a length serves kernels that
-// wrap at most half of its window.  Prefetching the next CTA's samples gained
-// 8 % at 16384 points, 3 % at 8192 and lost 4 % at 4096.
-int os_points(int64_t nout, int64_t count, int64_t nb) {
+// Transform length of the float32 blocks.  A non-finite or loud sample reaches
+// every output of the two blocks that share its transform (its rounding error,
+// where it is finite).  Two blocks of N points span 2 N - (nb - 1) samples, so
+// the lengths with 2 N <= Lb keep that within fewer than Lb samples, the window
+// of one block of os_length.  Among them the one whose waves of CTAs take the
+// least time (so a signal's last bits depend on how many share the call): `us`
+// is one full wave (148 SMs x resident CTAs), measured on 32 and 64 signals of
+// 2^20 (33 taps: 2048 points 0.080 ms, 4096 0.085; 513 taps: 4096 points 0.171,
+// 8192 0.205, 16384 0.261 ms; 4097 taps: 8192 points 0.349, 16384 0.306 ms); a
+// length serves kernels that wrap at most half of its window.  Prefetching the
+// next CTA's samples gained 8 % at 16384 points, 3 % at 8192 and lost 4 % at
+// 4096.
+int os_points(int64_t Lb, int64_t nout, int64_t count, int64_t nb) {
   static const struct {
     int n, resident;
     double us;
-  } kRows[] = {{4096, 4, 10.7}, {8192, 2, 13.7}, {16384, 1, 16.4}};
-  int best = 16384;
+  } kRows[] = {{2048, 8, 10.0}, {4096, 4, 10.7}, {8192, 2, 13.7}, {16384, 1, 16.4}};
+  int best = 0;
   double cost = 0;
   for (const auto& r : kRows) {
-    if (2 * (nb - 1) > r.n) continue;
+    if (2 * r.n > Lb || 2 * (nb - 1) > r.n) continue;
     const int64_t B = r.n - (nb - 1), pairs = count * (((nout + B - 1) / B + 1) / 2), wave = 148 * r.resident;
     const double c = double((pairs + wave - 1) / wave) * r.us;
-    if (cost == 0 || c < cost) {
+    if (best == 0 || c < cost) {
       cost = c;
       best = r.n;
     }
@@ -430,11 +437,11 @@ static gfft_status convolve_real_dev(int prec, R* dst, int64_t dst_dist, const R
   using C = Cx<R>;
   const int64_t L = na + nb - 1;
   // long signals: overlap-save blocks (same linear convolution, transforms
-  // of 2^12..2^15 points instead of one of NextPow2(na + nb - 1))
+  // of 2^11..2^14 points instead of one of NextPow2(na + nb - 1))
   const int64_t Lb = os_length<R>(na, nb);
   if constexpr (sizeof(R) == 4) {
     if (Lb) {
-      const int N = os_points(L, count, nb);
+      const int N = os_points(Lb, L, count, nb);
       gfft_plan* tp = nullptr;  // its W_N table
       gfft_status s = cached_plan(prec, N, &tp);
       if (s != GFFT_OK) return s;
@@ -444,7 +451,9 @@ static gfft_status convolve_real_dev(int prec, R* dst, int64_t dst_dist, const R
         const float2* tw = static_cast<const float2*>(tp->core.tw);
         const int64_t dd = count == 1 ? L : dst_dist;
         cudaError_t e;
-        if (N == 4096)
+        if (N == 2048)
+          e = launch_conv_pair<ConvRow2k, 8, false>(a, dst, na, a_dist, dd, L, count, b, int(nb), tw, hs, st);
+        else if (N == 4096)
           e = launch_conv_pair<ConvRow4k, 4, false>(a, dst, na, a_dist, dd, L, count, b, int(nb), tw, hs, st);
         else if (N == 8192)
           e = launch_conv_pair<ConvRow8k, 2, true>(a, dst, na, a_dist, dd, L, count, b, int(nb), tw, hs, st);

@@ -313,7 +313,10 @@ GFFT_API gfft_status gfft_correlate(int32_t precision, void* dst, int64_t dst_le
                                     const void* b, int64_t b_len, void* stream);
 /* ConvolveReal (convolve_real.go:9): real inputs (float32 for
  * GFFT_COMPLEX64, float64 for GFFT_COMPLEX128), FFT length
- * NextPow2(a_len + b_len - 1). */
+ * NextPow2(a_len + b_len - 1), or overlap-save blocks for long signals with
+ * a short kernel.  There a non-finite sample, or the rounding error of a loud
+ * stretch, reaches outputs fewer than W samples away, W the power of two of
+ * at least 8 (b_len - 1), 4096 <= W <= 32768. */
 GFFT_API gfft_status gfft_convolve_real(int32_t precision, void* dst, int64_t dst_len, const void* a, int64_t a_len,
                                         const void* b, int64_t b_len, void* stream);
 GFFT_API gfft_status gfft_convolve_host(int32_t precision, void* dst, int64_t dst_len, const void* a, int64_t a_len,
@@ -324,7 +327,9 @@ GFFT_API gfft_status gfft_convolve_real_host(int32_t precision, void* dst, int64
                                              int64_t a_len, const void* b, int64_t b_len);
 /* ConvolveReal of `count` signals (a_len reals, a_dist apart) with one kernel
  * b, results of a_len + b_len - 1 reals dst_dist apart: the reference's
- * per-signal ConvolveReal loop as one batched computation. */
+ * per-signal ConvolveReal loop as one batched computation.  The length of
+ * the float32 overlap-save blocks follows the count too, so a signal's last
+ * bits may differ between one call for it and a batch that holds it. */
 GFFT_API gfft_status gfft_convolve_real_batch(int32_t precision, void* dst, int64_t dst_dist, const void* a,
                                               int64_t a_len, int64_t a_dist, int64_t count, const void* b,
                                               int64_t b_len, void* stream);
