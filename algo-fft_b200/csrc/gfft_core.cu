@@ -5,6 +5,7 @@
 #include <cstdlib>
 #include <cstdio>
 #include <mutex>
+#include <new>
 #include <vector>
 #include "gfft_internal.h"
 #include "gfft_math.cuh"
@@ -394,6 +395,20 @@ static gfft_status init_pair(PlanCore* c, const PairKernel* k) {
     const ThreePassKernel* f = find_threepass(c->prec, c->n, -1);
     const ThreePassKernel* i = find_threepass(c->prec, c->n, +1);
     if (f && i && f->n1 == k->n1 && f->m1 == k->m1) s = init_threepass(c, f, i, k);
+    if (s == GFFT_OK && k->te) {
+      const TwoPassKernel* tf = find_twopass(c->prec, c->n, -1, k->te, k->emax);
+      const TwoPassKernel* ti = find_twopass(c->prec, c->n, +1, k->te, k->emax);
+      if (!tf || !ti) {
+        set_error("no scalar two-pass kernels beside the packed-pair split");
+        return GFFT_ERR_NOT_IMPLEMENTED;
+      }
+      c->sub = new (std::nothrow) PlanCore;
+      if (!c->sub) return GFFT_ERR_OUT_OF_MEMORY;
+      c->sub->prec = c->prec;
+      c->sub->n = c->n;
+      c->sub->device = c->device;
+      s = init_twopass(c->sub, tf, ti);
+    }
   } else {
     const TwoPassKernel* f = find_twopass(c->prec, c->n, -1, k->te, k->emax);
     const TwoPassKernel* i = find_twopass(c->prec, c->n, +1, k->te, k->emax);
@@ -638,10 +653,9 @@ gfft_status core_init(PlanCore* c, int prec, int64_t n, int device, int strategy
 }
 
 unsigned core_device_status(const PlanCore* c) {
-  if (!c->status) return 0;
   unsigned v = 0;
-  if (cudaMemcpy(&v, c->status, sizeof v, cudaMemcpyDeviceToHost) != cudaSuccess) return 0;
-  return v;
+  if (c->status && cudaMemcpy(&v, c->status, sizeof v, cudaMemcpyDeviceToHost) != cudaSuccess) v = 0;
+  return v || !c->sub ? v : core_device_status(c->sub);
 }
 
 void core_free(PlanCore* c) {

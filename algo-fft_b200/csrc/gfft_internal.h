@@ -106,6 +106,7 @@ struct PlanCore {
   int64_t gn1 = 0, gn2 = 0;
   bool mixc = false;  // two passes on the compiled mixed-radix column tiles
   bool mixr = false;  // one pass on the compiled tiles in rows mode (Algo::Generic)
+  // packed pairs in three passes: the length's scalar two-pass plan, or null;
   // Bluestein: chirps and filters per direction, sub-plan of length bm;
   // bsm: bm = gn1 x gn2 on the compiled mixed-radix tiles (tw1 = W_gn1,
   // tw2 = W_gn2, bt_* = W_bm split)

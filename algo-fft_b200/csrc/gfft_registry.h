@@ -55,8 +55,9 @@ struct L2PipeKernel {
 };
 
 // Packed-pair kernels of a complex64 length: two passes N1 x M1 (m2 = 0) or
-// three N1 x M1 x M2.  te / emax name the scalar two-pass tile that serves
-// buffers the 16-byte accesses cannot (three passes: the plain k_tp3).
+// three N1 x M1 x M2.  te / emax name the scalar two-pass tile of the length:
+// of two passes it serves buffers the 16-byte accesses cannot; beside three
+// passes it is a plan of its own for the allocation-free entry (te = 0: none).
 struct PairPassParams;
 struct PairKernel {
   int n1, m1, m2, te, emax;

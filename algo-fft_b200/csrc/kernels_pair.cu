@@ -128,20 +128,21 @@ PairKernel first_only(int te, int emax) {
                     {&launch_first<N1, N2, -1>, &launch_first<N1, N2, 1>}};
 }
 template <int N1, int M1, int M2>
-PairKernel three_pass() {
-  return PairKernel{N1, M1, M2, 0, 0, last_prefix<N1, Tile<N1>::E>(), false,
+PairKernel three_pass(int te = 0, int emax = 0) {
+  return PairKernel{N1, M1, M2, te, emax, last_prefix<N1, Tile<N1>::E>(), false,
                     {&launch_tp3<N1, M1, M2, -1>, &launch_tp3<N1, M1, M2, 1>}};
 }
 
 }  // namespace
 
 // One per length; te / emax: the scalar tile for buffers off 16 bytes (the
-// fastest scalar variant of the length).
+// fastest scalar variant of the length).  2^21 is the longest that the
+// allocation-free entry holds, so its plan has two-pass tables too.
 const PairKernel* find_pair(int64_t n) {
   static const PairKernel k[] = {
       two_pass<128, 256>(4096, 16),  two_pass<256, 256>(8192, 32),   first_only<256, 512>(8192, 32),
       first_only<512, 512>(8192, 32),  first_only<512, 1024>(8192, 32),  two_pass<1024, 1024>(8192, 16),
-      three_pass<128, 128, 128>(),   three_pass<256, 128, 128>(),    three_pass<256, 256, 128>(),
+      three_pass<128, 128, 128>(8192, 16), three_pass<256, 128, 128>(),    three_pass<256, 256, 128>(),
       three_pass<256, 256, 256>()};
   for (const PairKernel& e : k)
     if (int64_t(e.n1) * e.m1 * (e.m2 ? e.m2 : 1) == n) return &e;
