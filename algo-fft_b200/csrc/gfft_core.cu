@@ -617,7 +617,8 @@ gfft_status core_init(PlanCore* c, int prec, int64_t n, int device, int strategy
   const bool want_bluestein = strategy == GFFT_KERNEL_BLUESTEIN;
   if (pow2 && n <= max_single && !want_twopass && !want_bluestein) return init_pow2(c, default_ept(prec, n));
   if (pow2 && prec == kC64 && !want_single && !want_bluestein) {
-    if (const PairKernel* k = find_pair(n)) return init_pair(c, k);
+    const PairKernel* k = find_pair(n);
+    if (k && !(want_twopass && k->m2)) return init_pair(c, k);
   }
   if (pow2 && !want_single && strategy != GFFT_KERNEL_BLUESTEIN) {
     const TwoPassKernel* f = find_twopass(prec, n, -1, prec == kC64 ? 8192 : 4096, prec == kC64 ? 16 : 8);
