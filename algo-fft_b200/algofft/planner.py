@@ -218,9 +218,10 @@ def load_records(path: str = DEFAULT_DATA) -> list[dict]:
 
 def design(records: list[dict]):
     """X (rows x D raw features), y (log ns per element), owner shape index,
-    and the token of each row.  Variants without features (the L2-pipelined
-    two-pass, an autotuner candidate only) are left out, as plan creation
-    leaves them out of the model's candidates."""
+    and the token of each row.  Variants without features are left out, as
+    plan creation leaves them out of the model's candidates: the L2-pipelined
+    two-pass (an autotuner candidate only) and the packed-pair kernels (taken
+    without the model where they exist)."""
     X, y, owner, toks = [], [], [], []
     for i, r in enumerate(records):
         for tok, ms in r["times"].items():
