@@ -99,12 +99,13 @@ ColFn pick(int64_t L) {
 // 2.5-4.5e-7.  In long runs the power cap holds the clock near 1.6 GHz, so the
 // tiles with the fewest stages win (512 rows: 32 x 16).  4096 rows as two passes
 // of 64 through a workspace measured slower (1040-1085 us) than the one-pass
-// tile in place.  A length has one tile shape, so an array's result does not
-// depend on its batch.
+// tile in place.  128 rows stay on the scalar tile (16 x 16 in pairs: 64 x 128 x
+// 2048 91 -> 96 us, 8 x 128^3 136 -> 143).  A length has one tile shape, so an
+// array's result does not depend on its batch; the price is on one small array
+// of 2048 rows (512 columns: 12.3 -> 14.4 us).
 template <int L> struct PairTile;
 template <> struct PairTile<32> { static constexpr int E = 8, NP = 16, MB = 8; };
 template <> struct PairTile<64> { static constexpr int E = 8, NP = 16, MB = 8; };
-template <> struct PairTile<128> { static constexpr int E = 16, NP = 16, MB = 4; };
 template <> struct PairTile<256> { static constexpr int E = 16, NP = 8, MB = 4; };
 template <> struct PairTile<512> { static constexpr int E = 32, NP = 8, MB = 3; };
 template <> struct PairTile<1024> { static constexpr int E = 16, NP = 4, MB = 2; };
@@ -155,7 +156,6 @@ cudaError_t exec_pair_cols(const PairColsParams& p, int64_t n, int64_t count, cu
   switch (n) {
     case 32: return launch_pair_cols<32, DIR>(p, count, st);
     case 64: return launch_pair_cols<64, DIR>(p, count, st);
-    case 128: return launch_pair_cols<128, DIR>(p, count, st);
     case 256: return launch_pair_cols<256, DIR>(p, count, st);
     case 512: return launch_pair_cols<512, DIR>(p, count, st);
     case 1024: return launch_pair_cols<1024, DIR>(p, count, st);
@@ -172,7 +172,7 @@ bool pow2_cols_supported(int64_t n) { return n >= 2 && n <= 4096 && (n & (n - 1)
 cudaError_t exec_pow2_cols(int prec, int dir, void* dst, const void* src, int64_t count, int64_t dist, int64_t ncols,
                            int64_t pitch, const void* tw_n, int64_t n, cudaStream_t st) {
   // pairs: 16-byte rows throughout, and row offsets of a tile within 32 bits
-  if (prec == kC64 && n >= 32 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0 &&
+  if (prec == kC64 && n >= 32 && n != 128 && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0 &&
       ((ncols | pitch | dist) & 1) == 0 && ncols <= pitch && pitch < (int64_t(1) << 32) / n) {
     PairColsParams p{};
     p.src = static_cast<const float4*>(src);
