@@ -66,7 +66,7 @@ __device__ __forceinline__ void gen_stage(const C* in, C* out, const C* gin, C* 
     C v[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      if constexpr (GI) v[r] = ld_stream(gin + i + r * nb);
+      if constexpr (GI) v[r] = ld_evict(gin + i + r * nb);
       else v[r] = in[gpad(i + r * nb)];
     }
     int q;
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(1024) k_gen_cols(const C* src, C* dst, int64_t
     C v = C{0, 0};
     if (valid && col0 + c < ncols) {
       const C* p = in + int64_t(row) * pitch + col0 + c;
-      v = MODE == GEN_PASS1 ? ld_stream(p) : __ldcg(p);
+      v = MODE == GEN_PASS1 ? ld_evict(p) : __ldcg(p);
     }
     base[c * s.stride + gpad(row)] = v;
   }

@@ -267,18 +267,27 @@ __device__ __forceinline__ void prefetch_range(const void* p, int64_t bytes, int
   }
 }
 
-// Loads stay at the default eviction priority of L2: evict-first loads lost the
-// lines that several CTAs share parts of (column tiles, ragged rows) before
-// all of them had read theirs (256 transforms of 2^18: 400 -> 379 us, 4096 of
-// 10000 points: 202 -> 185 us with the default).
+// Input reads at the default eviction priority of L2, or evict-first.  Both
+// lose somewhere.  Evict-first drops lines that several CTAs share parts of
+// before all of them have read theirs (256 transforms of 2^18 400 us, 379 with
+// the default; 4096 of 10000 points 202, 185).  The default lets an input that
+// is read once push out what the next pass or the store is about to touch
+// (69042 rows of 243 points 66 us, 59.6 evict-first; an uneven batch of 120
+// transforms, about as large as L2, 181, 162).  So the column tiles of the
+// power-of-two passes and rows beyond 56 KB take the default; where the size
+// of the batch decides, the kernel exists in both forms.
 __device__ __forceinline__ float2 ld_stream(const float2* p) { return __ldcg(p); }
 __device__ __forceinline__ double2 ld_stream(const double2* p) { return __ldcg(p); }
-// Evict-first, for whole lines that one CTA reads once: the single-pass
-// kernel, whose next inputs are prefetched into L2 (16384 transforms of 4096
-// points: 199 against 201 us), and the column tiles of N-D axes (4096 x 4096
-// images: 1071 against 1105 us).
+// Evict-first also in the single-pass kernel, whose next inputs are prefetched
+// into L2 (16384 transforms of 4096 points: 199 against 201 us), and the column
+// tiles of N-D axes (4096 x 4096 images: 1071 against 1105 us).
 __device__ __forceinline__ float2 ld_evict(const float2* p) { return __ldcs(p); }
 __device__ __forceinline__ double2 ld_evict(const double2* p) { return __ldcs(p); }
+template <bool EVICT, typename C>
+__device__ __forceinline__ C ld_in(const C* p) {
+  if constexpr (EVICT) return ld_evict(p);
+  else return ld_stream(p);
+}
 __device__ __forceinline__ void st_stream(float2* p, float2 v) { __stcs(p, v); }
 __device__ __forceinline__ void st_stream(double2* p, double2 v) { __stcs(p, v); }
 

@@ -55,6 +55,7 @@ struct MixBsParams {
   int64_t tiles;      // batch mode: column tiles per transform; item mode: CTAs
   double scale;       // batch mode: output scale (1/n for the inverse)
   int inv;            // item mode: 1 for the inverse (conjugate tables, 1/n)
+  bool evict = false;  // host: BSK_IN reads x evict-first
   const MixBsItem* items = nullptr;
   const int32_t* blk = nullptr;
   const void* tab = nullptr;
@@ -67,7 +68,7 @@ __device__ __forceinline__ C bs_chirp(const C* w, int64_t m, int inv) {
   return v;
 }
 
-template <typename C>
+template <typename C, bool EVICT>
 struct MixBsIn {
   static constexpr bool kLoad = true, kStore = false;
   const C* x;
@@ -76,7 +77,7 @@ struct MixBsIn {
   int inv;
   __device__ __forceinline__ C load(int row, int c) const {
     const int64_t m = int64_t(row) * pitch + col0 + c;
-    return m < n ? cmul(ld_stream(x + m), bs_chirp(w, m, inv)) : C{0, 0};
+    return m < n ? cmul(ld_in<EVICT>(x + m), bs_chirp(w, m, inv)) : C{0, 0};
   }
 };
 
@@ -122,7 +123,7 @@ struct MixBsOut {
 
 // One CTA per column tile of one transform (batch mode: blockIdx =
 // transform * tiles + tile; item mode: items[blk[blockIdx]]).
-template <typename C, typename SC, int NC, int KIND, int MINB = 1, int TT = 0>
+template <typename C, typename SC, int NC, int KIND, int MINB = 1, int TT = 0, bool EVICT = false>
 __global__ void __launch_bounds__(MixTile<SC, NC, TT>::TPB, MINB) k_mix_bs(MixBsParams p) {
   if constexpr (KIND != BSK_OUT) asm volatile("griddepcontrol.launch_dependents;");
   if constexpr (KIND != BSK_IN) asm volatile("griddepcontrol.wait;" ::: "memory");  // the pass before this one
@@ -167,8 +168,8 @@ __global__ void __launch_bounds__(MixTile<SC, NC, TT>::TPB, MINB) k_mix_bs(MixBs
   C* scratch = static_cast<C*>(p.scratch);
   C v[TL::vmax()];
   if constexpr (KIND == BSK_IN) {
-    const MixBsIn<C> io{static_cast<const C*>(p.x) + off_x, w, n, ncols, col0, p.inv};
-    mix_stage<C, SC, TL, -1, 0, MIX_PASS1, MixBsIn<C>>(v, nullptr, nullptr, sh, t, c, active, tw, Re(1), bt,
+    const MixBsIn<C, EVICT> io{static_cast<const C*>(p.x) + off_x, w, n, ncols, col0, p.inv};
+    mix_stage<C, SC, TL, -1, 0, MIX_PASS1, MixBsIn<C, EVICT>>(v, nullptr, nullptr, sh, t, c, active, tw, Re(1), bt,
                                                        col0 + c, ncols, 0, io);
     C* yt = scratch + s + col0 * L;
     const int nv = int(ncols - col0 < NC ? ncols - col0 : NC);

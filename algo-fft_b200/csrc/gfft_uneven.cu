@@ -142,6 +142,7 @@ struct gfft_plan_uneven {
   MixBsItem* d_bsm_items = nullptr;
   std::vector<BsmChunk> bsm_chunks;
   int64_t bsm_buf = 0;  // elements of the largest chunk
+  bool evict = false;   // the first passes read the input evict-first
   // Recorded after every call's work: the next call, on whatever stream,
   // waits for it, so calls on one plan never overlap on the device (they
   // share the work buffers and queue counters above).
@@ -497,6 +498,15 @@ static gfft_status uneven_build(gfft_plan_uneven* p) {
     GFFT_CUDA(cudaMemcpy(p->d_bsm_items, p->bsm_items.data(), p->bsm_items.size() * sizeof(MixBsItem),
                          cudaMemcpyHostToDevice));
   }
+  // input, output and intermediates from half the size of the L2 to four times
+  // it (about 100 to 800 transforms of the mix): evict-first (120 transforms,
+  // 80 MB, 162 us, 179 with the default, 200 233 and 237, 450 394 and 398, 700
+  // the same); else the default (60 transforms 123 us, 127 evict-first, 1500 707
+  // and 712, 4000 1405 and 1415)
+  int64_t moved = 2 * p->total + p->mix_scratch + 2 * p->bsm_buf;
+  for (const Group& g : p->groups) moved += 2 * int64_t(g.items.size()) * g.M;
+  moved *= int64_t(es);
+  p->evict = moved >= int64_t(64) << 20 && moved <= int64_t(512) << 20;
   GFFT_CUDA(cudaMalloc(&p->counters, 2 * sizeof(unsigned)));
   GFFT_CUDA(cudaStreamCreateWithFlags(&p->cap, cudaStreamNonBlocking));
   for (int k = 0; k < gfft_plan_uneven::kSide; ++k) {
@@ -559,6 +569,7 @@ static gfft_status run_bsm(gfft_plan_uneven* p, C* dst, const C* src, cudaStream
       bp.items = p->d_bsm_items;
       bp.blk = bl.d_blk;
       bp.tab = p->tab;
+      bp.evict = p->evict;
       e = exec_mix_bs(p->prec, bl.kind, bl.L, bp, bl.blocks, s);
       if (e != cudaSuccess) break;
     }
@@ -587,9 +598,9 @@ static gfft_status run_group(gfft_plan_uneven* p, Group& g, C* dst, const C* src
     bt.shift = g.plan->bt_shift;
     const cudaError_t e =
         g.bluestein ? exec_bluestein_tp_items(p->prec, g.M, DIR, src, dst, g.d_items, rows, p->tab, g.plan->tw1,
-                                              g.plan->tw2, bt, scratch, work, s)
+                                              g.plan->tw2, bt, scratch, work, p->evict, s)
                     : exec_twopass_items(p->prec, g.M, DIR, src, dst, g.d_items, rows, g.plan->tw1, g.plan->tw2, bt,
-                                         scratch, s);
+                                         scratch, p->evict, s);
     cudaFreeAsync(scratch, s);
     GFFT_CUDA(e);
     return GFFT_OK;

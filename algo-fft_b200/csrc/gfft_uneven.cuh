@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(1024) k_uneven(const C* src, C* dst, const Une
     C* out = dst + it.off;
     if (!d.bluestein) {
       if (d.s.nst == 0) {  // length 1
-        for (int e = tid; e < L; e += nthr) st_stream(out + e, ld_stream(in + e));
+        for (int e = tid; e < L; e += nthr) st_stream(out + e, ld_evict(in + e));
       } else {
         // first stage from HBM, last stage to HBM
         gen_fft_io<DIR>(x, x + d.s.half, in, out, Re(1.0 / double(L)), d.s, t, W);
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(1024) k_uneven(const C* src, C* dst, const Une
       const C* ch = tab + d.chirp;
       const C* F = tab + d.filt;
       for (int e = tid; e < L; e += nthr)
-        x[gpad(e)] = e < n ? cmul(ld_stream(in + e), chirp_dir<DIR>(__ldg(ch + e))) : C{0, 0};
+        x[gpad(e)] = e < n ? cmul(ld_evict(in + e), chirp_dir<DIR>(__ldg(ch + e))) : C{0, 0};
       __syncthreads();
       C* y = gen_fft<-1>(x, x + d.s.half, d.s, t, W);
       C* other = y == x ? x + d.s.half : x;
@@ -109,7 +109,7 @@ __global__ void k_big_gather(C* work, int64_t M, const C* src, const BigItem* it
     const BigItem it = items[r];
     C v{0, 0};
     if (m < it.n) {
-      v = ld_stream(src + it.off + m);
+      v = ld_evict(src + it.off + m);
       if (bluestein) v = cmul(v, chirp_dir<DIR>(tab[it.chirp + m]));
     }
     work[e] = v;

@@ -37,14 +37,14 @@ __device__ __forceinline__ C chirp_of(const C* w, int64_t m) {
 }
 
 // chirp-weighted, zero-padded input: m = row * N2 + col0 + c
-template <typename C, int UDIR>
+template <typename C, int UDIR, bool EVICT>
 struct BsChirpIn {
   const C* x;  // this transform's input
   const C* w;
   int64_t n, n2, col0;
   __device__ __forceinline__ C load(int row, int c) const {
     const int64_t m = int64_t(row) * n2 + col0 + c;
-    return m < n ? cmul(ld_stream(x + m), chirp_of<UDIR>(w, m)) : C{0, 0};
+    return m < n ? cmul(ld_in<EVICT>(x + m), chirp_of<UDIR>(w, m)) : C{0, 0};
   }
 };
 
@@ -75,6 +75,7 @@ struct BsTpParams {
   BigTwiddle bt;     // W_M
   int64_t n, idist, odist;
   double inv_m, scale;  // items: the scale is 1/n for the inverse, else 1
+  bool evict;           // host: which form of the first pass
 };
 
 // One transform's buffers and parameters.
@@ -102,11 +103,13 @@ __device__ __forceinline__ BsRow<C> bs_row(const BsTpParams& p, int64_t b) {
 
 // Plain transform of an item of length M: reads and writes it in place in
 // the packed batch (uneven groups of one large length).
-template <typename C>
+template <typename C, bool EVICT>
 struct ItemIn {
   const C* x;
   int64_t n2, col0;
-  __device__ __forceinline__ C load(int row, int c) const { return ld_stream(x + int64_t(row) * n2 + col0 + c); }
+  __device__ __forceinline__ C load(int row, int c) const {
+    return ld_in<EVICT>(x + int64_t(row) * n2 + col0 + c);
+  }
 };
 
 template <typename C>
@@ -118,7 +121,8 @@ struct ItemOut {
 
 enum { BS_FWD1 = 0, BS_MID = 1, BS_INV2 = 2, PL_1 = 3, PL_2 = 4 };
 
-template <typename C, int N1, int EPT1, int NC1, int N2, int EPT2, int NC2, int KIND, int UDIR>
+// EVICT: the first pass reads the input evict-first.
+template <typename C, int N1, int EPT1, int NC1, int N2, int EPT2, int NC2, int KIND, int UDIR, bool EVICT = false>
 __global__ void __launch_bounds__(TwoPass<C, N1, EPT1, NC1, N2, EPT2, NC2, -1>::TPB,
                                   TwoPass<C, N1, EPT1, NC1, N2, EPT2, NC2, -1>::MIN_BLOCKS)
 k_bs_tp(BsTpParams p, int64_t b0) {
@@ -137,9 +141,9 @@ k_bs_tp(BsTpParams p, int64_t b0) {
     const bool active = tid < S1::TPB;
     const int c = tid % NC1, t = tid / NC1;
     const BsRow<C> rw = bs_row<C, UDIR>(p, b0 + bl);
-    const ItemIn<C> io{rw.x, N2, col0};
+    const ItemIn<C, EVICT> io{rw.x, N2, col0};
     C* y = scratch + bl * TP::N;
-    col_stage<C, N1, EPT1, NC1, UDIR, 1, LOAD_FN, OUT_SMEM_TWIDDLE, N2, 0, false, ItemIn<C>>(
+    col_stage<C, N1, EPT1, NC1, UDIR, 1, LOAD_FN, OUT_SMEM_TWIDDLE, N2, 0, false, ItemIn<C, EVICT>>(
         v, nullptr, nullptr, sh, t, c, active, static_cast<const C*>(p.tw1), Re(1), p.bt, int64_t(col0 + c), 0, io);
     for (int e = tid; e < N1 * NC1; e += TP::TPB) {
       const int cc = e / N1, row = e % N1;
@@ -161,9 +165,9 @@ k_bs_tp(BsTpParams p, int64_t b0) {
     const bool active = tid < S1::TPB;
     const int c = tid % NC1, t = tid / NC1;
     const BsRow<C> rw = bs_row<C, UDIR>(p, b0 + bl);
-    const BsChirpIn<C, UDIR> io{rw.x, rw.w, rw.n, N2, col0};
+    const BsChirpIn<C, UDIR, EVICT> io{rw.x, rw.w, rw.n, N2, col0};
     C* y = scratch + bl * TP::N;
-    col_stage<C, N1, EPT1, NC1, -1, 1, LOAD_FN, OUT_SMEM_TWIDDLE, N2, 0, false, BsChirpIn<C, UDIR>>(
+    col_stage<C, N1, EPT1, NC1, -1, 1, LOAD_FN, OUT_SMEM_TWIDDLE, N2, 0, false, BsChirpIn<C, UDIR, EVICT>>(
         v, nullptr, nullptr, sh, t, c, active, static_cast<const C*>(p.tw1), Re(1), p.bt, int64_t(col0 + c), 0,
         io);
     for (int e = tid; e < N1 * NC1; e += TP::TPB) {
@@ -222,7 +226,8 @@ struct BsTpKernel {
   int64_t m;
   int n1;
   int tpb, smem;
-  const void* fn[10];  // fused Bluestein passes (UDIR -1, +1; the last of the transposed split), item passes
+  const void* fn[14];  // fused Bluestein passes (UDIR -1, +1; the last of the transposed split), item passes, the
+                       // first passes evict-first
   cudaError_t (*run)(const BsTpParams& p, int udir, int64_t count, void* scratch, void* work, cudaStream_t st);
   cudaError_t (*run_plain)(const BsTpParams& p, int udir, int64_t count, void* scratch, cudaStream_t st);
 };
@@ -240,9 +245,17 @@ struct BsTpOf {
   using TP = TwoPass<C, N1, A::EPT, A::NC, N2, B::EPT, B::NC, -1>;
   // the inverse FFT's split N2 x N1: its second pass runs columns of N1
   using TS = TwoPass<C, N2, B::EPT, B::NC, N1, A::EPT, A::NC, -1>;
-  template <int KIND, int UDIR>
+  template <int KIND, int UDIR, bool EVICT = false>
   static const void* fn() {
-    return reinterpret_cast<const void*>(&k_bs_tp<C, N1, A::EPT, A::NC, N2, B::EPT, B::NC, KIND, UDIR>);
+    return reinterpret_cast<const void*>(&k_bs_tp<C, N1, A::EPT, A::NC, N2, B::EPT, B::NC, KIND, UDIR, EVICT>);
+  }
+  template <int KIND, int UDIR>
+  static void first(const BsTpParams& p, int64_t b0, int64_t nb, cudaStream_t st) {
+    const unsigned grid = unsigned(nb * TP::TILES1);
+    if (p.evict)
+      k_bs_tp<C, N1, A::EPT, A::NC, N2, B::EPT, B::NC, KIND, UDIR, true><<<grid, TP::TPB, TP::SMEM, st>>>(p, b0);
+    else
+      k_bs_tp<C, N1, A::EPT, A::NC, N2, B::EPT, B::NC, KIND, UDIR, false><<<grid, TP::TPB, TP::SMEM, st>>>(p, b0);
   }
   template <int UDIR>
   static const void* fn_inv2() {
@@ -257,8 +270,7 @@ struct BsTpOf {
     q.tw2 = p.tw1;
     for (int64_t b0 = 0; b0 < count; b0 += chunk) {
       const int64_t nb = std::min(chunk, count - b0);
-      k_bs_tp<C, N1, A::EPT, A::NC, N2, B::EPT, B::NC, BS_FWD1, UDIR>
-          <<<unsigned(nb * TP::TILES1), TP::TPB, TP::SMEM, st>>>(p, b0);
+      first<BS_FWD1, UDIR>(p, b0, nb, st);
       k_bs_tp<C, N1, A::EPT, A::NC, N2, B::EPT, B::NC, BS_MID, UDIR>
           <<<unsigned(nb * TP::TILES2), TP::TPB, TP::SMEM, st>>>(p, b0);
       k_bs_tp<C, N2, B::EPT, B::NC, N1, A::EPT, A::NC, BS_INV2, UDIR>
@@ -273,8 +285,7 @@ struct BsTpOf {
     const int64_t chunk = std::max<int64_t>(1, std::min<int64_t>(count, (int64_t(256) << 20) / (TP::N * int64_t(sizeof(C)))));
     for (int64_t b0 = 0; b0 < count; b0 += chunk) {
       const int64_t nb = std::min(chunk, count - b0);
-      k_bs_tp<C, N1, A::EPT, A::NC, N2, B::EPT, B::NC, PL_1, UDIR>
-          <<<unsigned(nb * TP::TILES1), TP::TPB, TP::SMEM, st>>>(p, b0);
+      first<PL_1, UDIR>(p, b0, nb, st);
       k_bs_tp<C, N1, A::EPT, A::NC, N2, B::EPT, B::NC, PL_2, UDIR>
           <<<unsigned(nb * TP::TILES2), TP::TPB, TP::SMEM, st>>>(p, b0);
       const cudaError_t e = cudaGetLastError();
@@ -319,6 +330,10 @@ void reg() {
   k.fn[7] = O::template fn<PL_2, -1>();
   k.fn[8] = O::template fn<PL_1, +1>();
   k.fn[9] = O::template fn<PL_2, +1>();
+  k.fn[10] = O::template fn<BS_FWD1, -1, true>();
+  k.fn[11] = O::template fn<BS_FWD1, +1, true>();
+  k.fn[12] = O::template fn<PL_1, -1, true>();
+  k.fn[13] = O::template fn<PL_1, +1, true>();
   k.run = &O::run;
   k.run_plain = &O::run_plain;
   table().push_back(k);
@@ -403,12 +418,16 @@ cudaError_t exec_bluestein_tp(int prec, int64_t M, const void* src, void* dst, i
   p.odist = odist;
   p.inv_m = 1.0 / double(M);
   p.scale = scale;
+  // input, output and two intermediates up to twice the L2: evict-first (16 x
+  // 131071: 59.9 us, 62.5 with the default; 64 x 65521 107.6, 108.8); beyond,
+  // the default (64 x 131071 206, 208; 256 x 65521 375, 378)
+  p.evict = count * 2 * (n + M) * int64_t(elem_bytes(prec)) <= int64_t(256) << 20;
   return k->run(p, -1, count, scratch, work, st);
 }
 
 cudaError_t exec_twopass_items(int prec, int64_t M, int dir, const void* src, void* dst, const BigItem* items,
                                int64_t rows, const void* tw1, const void* tw2, BigTwiddle bt, void* scratch,
-                               cudaStream_t st) {
+                               bool evict, cudaStream_t st) {
   cudaError_t e;
   const BsTpKernel* k = bs_tp_ready(prec, M, &e);
   if (!k) return e;
@@ -420,12 +439,13 @@ cudaError_t exec_twopass_items(int prec, int64_t M, int dir, const void* src, vo
   p.tw2 = tw2;
   p.bt = bt;
   p.inv_m = 1.0 / double(M);
+  p.evict = evict;
   return k->run_plain(p, dir, rows, scratch, st);
 }
 
 cudaError_t exec_bluestein_tp_items(int prec, int64_t M, int dir, const void* src, void* dst, const BigItem* items,
                                     int64_t rows, const void* tab, const void* tw1, const void* tw2, BigTwiddle bt,
-                                    void* scratch, void* work, cudaStream_t st) {
+                                    void* scratch, void* work, bool evict, cudaStream_t st) {
   cudaError_t e;
   const BsTpKernel* k = bs_tp_ready(prec, M, &e);
   if (!k) return e;
@@ -438,6 +458,7 @@ cudaError_t exec_bluestein_tp_items(int prec, int64_t M, int dir, const void* sr
   p.tw2 = tw2;
   p.bt = bt;
   p.inv_m = 1.0 / double(M);
+  p.evict = evict;
   return k->run(p, dir, rows, scratch, work, st);
 }
 

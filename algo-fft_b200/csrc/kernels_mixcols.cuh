@@ -97,17 +97,24 @@ inline cudaError_t launch_mix_bs_kernel(void (*kern)(MixBsParams), const MixBsPa
   return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
-template <typename C, typename CFG, int KIND>
-cudaError_t launch_mix_bs(const MixBsParams& p, int64_t blocks, cudaStream_t st) {
+template <typename C, typename CFG, int KIND, bool EVICT>
+cudaError_t launch_mix_bs_form(const MixBsParams& p, int64_t blocks, cudaStream_t st) {
   using SC = typename CFG::Sched;
   constexpr int NC = CFG::nc;
   using TL = MixTile<SC, NC, CFG::tt>;
   constexpr int smem = (KIND == BSK_OUT ? TL::ELEMS2 : TL::ELEMS1) * int(sizeof(C));
-  auto kern = &k_mix_bs<C, SC, NC, KIND, CFG::minb, CFG::tt>;
+  auto kern = &k_mix_bs<C, SC, NC, KIND, CFG::minb, CFG::tt, EVICT>;
   static const cudaError_t attr =
       smem > 48 * 1024 ? cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) : cudaSuccess;
   if (attr != cudaSuccess) return attr;
   return launch_mix_bs_kernel(kern, p, KIND, blocks, TL::TPB, smem, st);
+}
+
+template <typename C, typename CFG, int KIND>
+cudaError_t launch_mix_bs(const MixBsParams& p, int64_t blocks, cudaStream_t st) {
+  if constexpr (KIND == BSK_IN)
+    if (p.evict) return launch_mix_bs_form<C, CFG, KIND, true>(p, blocks, st);
+  return launch_mix_bs_form<C, CFG, KIND, false>(p, blocks, st);
 }
 
 // Whether a complex64 pass of the chain runs on packed pairs: tiles of 16
