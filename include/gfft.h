@@ -340,7 +340,9 @@ GFFT_API gfft_status gfft_convolve_real_batch(int32_t precision, void* dst, int6
  * plan per length.  A plan for `count` transforms of the given lengths
  * (1 .. 2^24 each), packed back to back: transform i starts at the sum of
  * the lengths before it.  Plan creation builds every twiddle, chirp and
- * Bluestein filter on the GPU. */
+ * Bluestein filter on the GPU.  Some kernels are chosen by how many transforms
+ * of a kind the plan has, so a transform's last bits may differ between plans
+ * that hold it among others. */
 typedef struct gfft_plan_uneven gfft_plan_uneven;
 GFFT_API gfft_status gfft_plan_uneven_new(gfft_plan_uneven** out, int32_t precision, int64_t count,
                                           const int64_t* lengths, const gfft_plan_options* opts);
