@@ -218,7 +218,8 @@ cudaError_t launch_conv_os(const void* a, void* dst, int64_t na, int64_t a_dist,
 // smallest power of two with at most an eighth of each window wrapped (L >= 8
 // (nb - 1)), else at most a quarter, at least 4096, at most 2^15 (float64:
 // 2^14, what one CTA transforms as L / 2 complex points); 0 = one transform of
-// the whole signal (short signals, long kernels).
+// the whole signal (short signals, long kernels).  In float32 it bounds how far
+// two blocks that share a transform may reach (os_points).
 template <typename R>
 int64_t os_length(int64_t na, int64_t nb) {
   const int64_t lmax = sizeof(R) == 4 ? 32768 : 16384;
@@ -436,8 +437,9 @@ static gfft_status convolve_real_dev(int prec, R* dst, int64_t dst_dist, const R
                                      int64_t count, const R* b, int64_t nb, cudaStream_t st) {
   using C = Cx<R>;
   const int64_t L = na + nb - 1;
-  // long signals: overlap-save blocks (same linear convolution, transforms
-  // of 2^11..2^14 points instead of one of NextPow2(na + nb - 1))
+  // long signals: overlap-save blocks (same linear convolution, transforms of
+  // 2^11..2^14 complex points, float64 2^12..2^14 reals, instead of one of
+  // NextPow2(na + nb - 1))
   const int64_t Lb = os_length<R>(na, nb);
   if constexpr (sizeof(R) == 4) {
     if (Lb) {

@@ -36,8 +36,10 @@ __device__ __forceinline__ Pair pair_table(const float2* t, unsigned k) {
   else return pair_of(f);
 }
 
-// v[r] *= b s^r, r < RS <= 32, from b, s and s4 = s^4 (both rounded from the
-// table, so no factor is more than three products away from it).
+// v[r] *= b s^r, r < RS <= 32, from b, s and s4 = s^4, each looked up: a factor
+// is at most RS / 4 + 2 rounded products away from them (RS / 4 - 2 for the
+// power of s4, two for that of s, two that join them with b; 6 at RS = 16, 10 at
+// 32), where powers of s alone would multiply its rounding error by r.
 template <int RS>
 __device__ __forceinline__ void pair_scale_powers(Pair* v, Pair b, Pair s, Pair s4) {
   Pair lo[4];
