@@ -153,7 +153,9 @@ __device__ __forceinline__ void mix_stage(C* v, const C* in, C* out, C* sh, int 
           v[q * RS + r] = io.load(row, c);
         } else if constexpr (FIRST) {
           const C* p = in + int64_t(row) * ip + c;
-          v[q * RS + r] = PASS == MIX_PASS1 ? ld_evict(p) : __ldcg(p);
+          // complex64 evict-first (332 of 50421 points 126 -> 124 us, and uneven
+          // batches), complex128 not (16 of 100000 points 26.7 us, 28.7 evict-first)
+          v[q * RS + r] = PASS == MIX_PASS1 ? ld_in<sizeof(C) == 8>(p) : __ldcg(p);
         } else {
           v[q * RS + r] = sh[TL::phys(row, c)];
         }
