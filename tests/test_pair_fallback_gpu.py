@@ -1,6 +1,5 @@
-"""Where packed-pair kernels do not run: a
-forced two-pass strategy takes two passes, and columns of 128 rows stay on the
-scalar tile."""
+"""Where packed-pair kernels do not run: a forced two-pass strategy takes two
+passes, and columns of 128 rows stay on the scalar tile."""
 import pytest
 
 import algofft
